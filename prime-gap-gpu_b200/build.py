@@ -51,6 +51,11 @@ def group_list() -> list[tuple[int, int]]:
     return [(int(a), int(b)) for a, b in re.findall(r"X\((\d+),\s*(\d+)\)", m.group(1))]
 
 
+def tc_list() -> list[int]:
+    m = re.search(r"#define PG_TC_LIST\(X\)(.*)", limbs_header())
+    return [int(v) for v in re.findall(r"X\((\d+)\)", m.group(1))]
+
+
 def headers() -> list[pathlib.Path]:
     return sorted(CSRC.glob("*.h")) + sorted(CSRC.glob("*.cuh")) + [ROOT / "include" / "primegap.h"]
 
@@ -65,6 +70,8 @@ def units() -> list[tuple[pathlib.Path, pathlib.Path, list[str]]]:
         out.append((CSRC / "pg_inst.cu", BUILD / f"pg_inst_{L}.o", [f"-DPG_LIMBS={L}"]))
     for T, LT in group_list():
         out.append((CSRC / "pg_ginst.cu", BUILD / f"pg_ginst_{T}x{LT}.o", [f"-DPG_GT={T}", f"-DPG_GLT={LT}"]))
+    for L in tc_list():
+        out.append((CSRC / "pg_tcinst.cu", BUILD / f"pg_tcinst_{L}.o", [f"-DPG_TCL={L}"]))
     return out
 
 

@@ -106,6 +106,46 @@ static double big_log(const Big &a) {
     return std::log(d) + std::log(2.0) * (double)bits;
 }
 
+// log2 of the positive a
+static double big_log2(const Big &a) {
+    double v = 0;
+    for (size_t i = a.size(), n = 0; i-- > 0 && n < 4; n++) v = v + std::ldexp((double)a[i], -32 * (int)n);
+    return std::log2(v) + 32.0 * (double)(a.size() - 1);
+}
+
+// floor(2^u / k) as words of out (k > 0), one bit at a time
+static bool big_pow2_div(uint32_t u, const Big &k, uint32_t *out, size_t words) {
+    std::memset(out, 0, words * 4);
+    Big r(k.size() + 1, 0);
+    for (uint32_t b = u + 1; b-- > 0;) {
+        uint32_t carry = b == u;  // the one set bit of 2^u
+        for (auto &w : r) {
+            const uint32_t t = w >> 31;
+            w = (w << 1) | carry;
+            carry = t;
+        }
+        bool ge = r.back() != 0;
+        if (!ge) {
+            ge = true;
+            for (size_t i = k.size(); i-- > 0;)
+                if (r[i] != k[i]) {
+                    ge = r[i] > k[i];
+                    break;
+                }
+        }
+        if (!ge) continue;
+        uint64_t borrow = 0;
+        for (size_t i = 0; i < r.size(); i++) {
+            const uint64_t d = (uint64_t)r[i] - (i < k.size() ? k[i] : 0u) - borrow;
+            r[i] = (uint32_t)d;
+            borrow = d >> 63;
+        }
+        if (b / 32 >= words) return false;
+        out[b / 32] |= 1u << (b % 32);
+    }
+    return true;
+}
+
 static std::vector<uint32_t> host_primes(uint32_t n) {  // all primes <= n
     std::vector<uint8_t> comp(n + 1, 0);
     std::vector<uint32_t> out;
@@ -481,8 +521,9 @@ int pg::slot_alloc(Slot &s, uint64_t nm_cap, uint64_t nodd_cap, uint64_t bm_cap,
         (rc = dalloc(b, &s.d_kstart, S)) || (rc = dalloc(b, &s.d_knext, S)) || (rc = dalloc(b, &s.d_gaps, S)) ||
         (rc = dalloc(b, &s.d_act0, S)) || (rc = dalloc(b, &s.d_act1, S)) || (rc = dalloc(b, &s.d_redo, S)) ||
         (rc = dalloc(b, &s.d_conf, S)) ||
-        (rc = dalloc(b, &s.d_sc, 1)) || (rc = dalloc(b, &s.d_win, win_cap)))
+        (rc = dalloc(b, &s.d_sc, 1 + (win_cap * 8 + sizeof(Scalars) - 1) / sizeof(Scalars))) || (rc = dalloc(b, &s.d_win, win_cap)))
         return rc;
+    s.d_wnext = reinterpret_cast<unsigned long long *>(s.d_sc + 1);
     PG_CUDA(cudaMallocHost((void **)&s.h_sc, sizeof(Scalars)));
     PG_CUDA(cudaMallocHost((void **)&s.h_ms, std::max<uint64_t>(nm_cap, 1) * 8));
     PG_CUDA(cudaMallocHost((void **)&s.h_wid, std::max<uint64_t>(nm_cap, 1) * 2));
@@ -513,6 +554,7 @@ void pg::slot_reset(Slot &s) {
     s.nm = 0;
     s.nodd = 0;
     s.L = 0;
+    s.tcL = 0;
     s.stride = 0;
     s.ext_window = 0;
     s.confirm = false;
@@ -564,8 +606,12 @@ int pg::slot_add(Slot &s, pg_job *j, uint64_t m_start, uint64_t m_inc) {
     s.h_win[wid] = j->win;
     if (s.parts.empty()) {
         s.L = j->L;
+        s.tcL = j->tcL;
         s.ext_window = p.ext_window;
     }
+    if (s.tcL != j->tcL) s.tcL = 0;
+    s.h_win[wid].side0 = 2 * s.nm;
+    s.h_win[wid].nsides = 2 * w.nm;
     s.stride = std::max(s.stride, j->cap);
     s.confirm = s.confirm || j->win.confirm_rounds >= 2;
     s.nm += w.nm;
@@ -712,6 +758,12 @@ static SearchArgs base_args(Slot &s) {
     return a;
 }
 
+// The persistent search of the slot's windows (first launch and resume).
+static cudaError_t launch_search(Slot &s) {
+    return s.search_tc ? launch_search_tc(s.tcL, s.search, s.tc_grid, s.st)
+                       : launch_search_persistent(s.L, s.search, s.grid, s.st);
+}
+
 // Finalize all sides and queue the copies back; the host reads n_redo in
 // slot_finish.
 static int enqueue_finalize(Slot &s, SearchArgs &a, uint32_t S) {
@@ -760,9 +812,19 @@ static int enqueue_windows(Slot &s, int form, uint32_t flags) {
             a.stop = s.d_stop;
             a.stopped = &s.d_sc->stopped;
         }
+        // a draining launch counts warps that leave one by one: the one-warp kernel
+        s.search_tc = s.tcL && !a.drain_lanes;
+        if (s.search_tc) {
+            a.win_next = s.d_wnext;
+            a.n_win = (uint32_t)s.parts.size();
+            a.failed = &s.d_sc->failed;
+            a.settle = s.tc_settle;
+            a.rounds = s.d_sc->rounds;
+            PG_CUDA(cudaMemsetAsync(s.d_wnext, 0, s.parts.size() * 8, s.st));
+        }
         s.search = a;
         PG_CUDA(record_ev(s.ev[3], s.st));
-        PG_CUDA(launch_search_persistent(s.L, a, s.grid, s.st));
+        PG_CUDA(launch_search(s));
         PG_CUDA(record_ev(s.ev[4], s.st));
         s.sst.kernel_launches++;
         s.sst.passes = 1;
@@ -817,7 +879,7 @@ int pg::slot_resume(Slot &s) {
     s.fin_active = false;
     const uint32_t S = 2 * s.nm;
     PG_CUDA(cudaMemsetAsync(&s.d_sc->stopped, 0, 4, s.st));
-    PG_CUDA(launch_search_persistent(s.L, s.search, s.grid, s.st));
+    PG_CUDA(launch_search(s));
     s.sst.kernel_launches++;
     s.sst.relaunches++;
     SearchArgs a = s.search;
@@ -826,6 +888,49 @@ int pg::slot_resume(Slot &s) {
     a.max_count = nullptr;
     a.stop = nullptr;
     return enqueue_finalize(s, a, S);
+}
+
+// CTAs of the tensor-core search for the slot's sides.  Every CTA tests 128
+// candidates at a time, the nearest of the sides still open, and c of them on
+// an SM take about 1 + 0.43 (c - 1) times as long per round as one (L = 23:
+// 3 800, 5 400, 6 900, 8 900 cycles a step at c = 1 .. 4).  A side takes
+// 1 / p tests on average, p = e^gamma ln(max_prime) / ln N, so a round of
+// `lanes` tests leaves a share exp(-p * lanes / open) of the open sides.  Many
+// sides want every CTA that fits; few sides want the shorter rounds, since
+// the deeper candidates of a fuller device are tested for nothing.  The CTAs
+// of a round end within a few per cent of each other, and those that end
+// first would refill with the next candidates of sides whose prime the others
+// are about to report, so with few rounds each CTA waits, at most an eighth of
+// its round, until the rounds begun before its own ended have ended too.
+static int tc_ctas(Slot &s) {
+    const int sms = s.parts[0].job->ctx->sms, most = tc_blocks_per_sm(s.tcL);
+    double tests = 0, sides = 0;
+    for (const WinPart &w : s.parts) {
+        const pg_job *j = w.job;
+        const double ln_n = j->T->k_log + std::log((double)w.m0 + 1);
+        sides += 2.0 * w.nm;
+        tests += 2.0 * w.nm * std::max(1.0, ln_n / (1.781 * std::log((double)std::max<uint64_t>(j->prm.max_prime, 3))));
+    }
+    const double per_side = tests / std::max(sides, 1.0);
+    int best = most;
+    s.tc_settle = 0;
+    double best_t = 1e300;
+    for (int c = most; c >= 1; c--) {
+        const double lanes = (double)c * sms * 128;
+        if (tests > 24 * lanes) break;  // throughput decides
+        double open = sides, rounds = 0;
+        while (open > 0.05 && rounds < 100) {
+            open *= std::exp(-lanes / (open * per_side));
+            rounds++;
+        }
+        const double t = rounds * (1 + 0.43 * (c - 1));
+        if (t < best_t) {
+            best_t = t;
+            best = c;
+            s.tc_settle = 8;
+        }
+    }
+    return sms * best;
 }
 
 int pg::slot_enqueue(Slot &s, int form, uint32_t flags, bool graph) {
@@ -837,6 +942,13 @@ int pg::slot_enqueue(Slot &s, int form, uint32_t flags, bool graph) {
     s.grid = search_grid(s.L, s.parts[0].job->ctx->device);
     const uint32_t wps = (flags >> 16) & 0xffu;  // warps per SM cap
     if (wps) s.grid = std::min(s.grid, s.parts[0].job->ctx->sms * (int)wps * 32 / PERSIST_THREADS);
+    if (s.tcL) {
+        s.tc_grid = tc_ctas(s);
+        if (wps) {  // another launch runs beside this one
+            s.tc_grid = std::max(1, std::min(s.tc_grid, s.parts[0].job->ctx->sms * (int)wps / 4));
+            s.tc_settle = 0;
+        }
+    }
     if (form == PG_SEARCH_PLAIN || !graph) return enqueue_windows(s, form, flags);
     // The persistent form's whole window (upload, sieves, search, finalize,
     // copies back) is captured as one CUDA graph and launched once; the slot
@@ -879,6 +991,7 @@ int pg::slot_finish(Slot &s, bool wait) {
         PG_CUDA(cudaStreamSynchronize(s.st));  // no wait when the caller saw the stream idle
         if (s.nm == 0) return PG_OK;
         if (!s.fin_active) {
+            if (s.search_tc && s.h_sc->failed) return fail(PG_ERR_CUDA, "search: a matrix instruction did not complete");
             if (s.h_sc->stopped) return SLOT_STOPPED;  // preempted before its queue ran out: slot_resume
             s.fin_active = true;
             s.fin_phase = 0;
@@ -1033,6 +1146,15 @@ static int job_build(pg_job *j) {
     j->win.k_log = T.k_log;
     j->win.confirm_merit = p.confirm_merit;
     j->win.confirm_rounds = p.confirm_merit > 0 ? (p.confirm_rounds ? p.confirm_rounds : 16u) : 0u;
+    j->tcL = 0;
+    if (!(j->L >> 16)) j->tcL = pick_tc(T.kbits, big_log2(T.K), p.max_m, 2ull * ((uint64_t)j->sly + p.ext_window));
+    if (j->tcL) {  // mu = floor(2^u / K), u = h + 8 (mu_off + 4): 8 bits more than T has
+        const uint32_t h = 32 * (j->tcL - 4);
+        const double t_log2 = 2 * (big_log2(T.K) + std::log2((double)p.max_m + 1)) + 2.31;
+        const uint32_t cols = (uint32_t)std::ceil((t_log2 + 8 - h) / 8);  // mu_off + 4
+        j->win.mu_off = (int32_t)cols - 4;
+        if (!big_pow2_div(h + 8 * cols, T.K, j->win.mu, TC_MU_WORDS)) j->tcL = 0;
+    }
     j->coprime.assign(p.d, 0);
     for (uint32_t r = 0; r < p.d; r++) j->coprime[r] = gcd64(r, p.d) == 1;
     // ---- window capacity

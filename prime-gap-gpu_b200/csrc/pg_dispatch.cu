@@ -5,6 +5,9 @@
 #include "pg_limbs.h"
 #include "pg_search.cuh"
 #include "pg_search_group.cuh"
+#include "pg_tc_search.cuh"
+
+#include <cmath>
 
 namespace pg {
 
@@ -14,6 +17,9 @@ PG_LIMB_LIST(PG_DECL)
 #define PG_GDECL(t, lt) PG_GDECLARE(t, lt)
 PG_GROUP_LIST(PG_GDECL)
 #undef PG_GDECL
+#define PG_TDECL(n) PG_TC_DECLARE(n)
+PG_TC_LIST(PG_TDECL)
+#undef PG_TDECL
 
 bool supported_limbs(uint32_t L) {
 #define PG_CASE(n) \
@@ -91,6 +97,48 @@ cudaError_t launch_search_persistent(uint32_t L, const SearchArgs &a, int grid, 
     if (L == PG_LAYOUT_GROUP(t, (t) * (lt))) return glaunch_search_persistent<t, lt>(a, grid, st);
     PG_GROUP_LIST(PG_GCASE)
 #undef PG_GCASE
+    return cudaErrorInvalidValue;
+}
+
+// The sizes the error bounds of pg_tc.cuh's step are stated for, with
+// n <= 2^n_log2, |X| < 2^x_log2, y < 2.22 n (2^1.16), T < 2^2.31 n^2, L words:
+//   y fits L words, z = m*T/n fits L + 1;
+//   the words of T and z left out (T_hi = T >> 32 (L-4); the correction reads
+//   z above 2^(32 (L-4))) weigh less than 2^-8: 2^(32 (L-4)) * |X| / K < 2^-8;
+//   the correction, at most |X| * m * 2^2.31 with relative error 2^-51.4, is
+//   off by less than 2^-5;
+//   m * 2 and |X| * 2 leave the 64-bit sums of the last line without a carry.
+uint32_t pick_tc(uint32_t kbits, double k_log2, uint64_t max_m, uint64_t max_x) {
+    if (max_m == 0 || max_m >= (1ull << 30) || max_x >= (1ull << 24)) return 0;
+    const double m_log2 = std::log2((double)max_m), x_log2 = std::log2((double)max_x);
+    const double n_log2 = std::log2((double)max_m + 1) + k_log2;
+    if (m_log2 + x_log2 > 44) return 0;
+    uint32_t best = 0;
+#define PG_TCASE(n) \
+    if (!best && 32.0 * (n) >= n_log2 + 1.17) best = n;
+    PG_TC_LIST(PG_TCASE)
+#undef PG_TCASE
+    if (!best) return 0;
+    if (n_log2 + m_log2 + 2.4 > 32.0 * (best + 1)) return 0;
+    if ((double)kbits - 1 < 32.0 * (best - 4) + x_log2 + 8) return 0;
+    return best;
+}
+
+int tc_blocks_per_sm(uint32_t tcL) {
+    int per = 0;
+#define PG_TCASE(n) \
+    if (tcL == n) per = tc_occupancy_t<n>();
+    PG_TC_LIST(PG_TCASE)
+#undef PG_TCASE
+    return per < 1 ? 1 : per;
+}
+
+cudaError_t launch_search_tc(uint32_t tcL, const SearchArgs &a, int grid, cudaStream_t st) {
+    if (a.n_act == 0) return cudaSuccess;
+#define PG_TCASE(n) \
+    if (tcL == n) return launch_search_tc_t<n>(a, grid, st);
+    PG_TC_LIST(PG_TCASE)
+#undef PG_TCASE
     return cudaErrorInvalidValue;
 }
 

@@ -99,6 +99,7 @@ struct Slot {
     uint32_t *d_conf = nullptr;  // per side: the k whose prime passed the record confirmation
     Scalars *d_sc = nullptr;
     WinInfo *d_win = nullptr;
+    unsigned long long *d_wnext = nullptr;  // queue heads of the tensor-core search (behind d_sc)
     // pinned host staging
     Scalars *h_sc = nullptr;
     uint64_t *h_ms = nullptr;
@@ -114,6 +115,8 @@ struct Slot {
     uint32_t nm = 0;       // m in the slot
     uint64_t nodd = 0;     // odd m in the slot
     uint32_t L = 0;        // operand layout of every window
+    uint32_t tcL = 0;      // operand words of the tensor-core search, 0 = some window cannot use it
+    bool search_tc = false;  // the search in flight runs on it
     uint32_t stride = 0;   // list stride (largest job capacity)
     uint32_t ext_window = 0;
     bool confirm = false;  // a window of the slot confirms the primes of its large gaps
@@ -127,7 +130,8 @@ struct Slot {
     bool fin_active = false;
     int fin_phase = 0;
     uint32_t fin_round = 0, fin_ext = 0;
-    int grid = 0;
+    int grid = 0, tc_grid = 0;
+    uint32_t tc_settle = 0;  // SearchArgs::settle
     bool busy = false;
     uint64_t ticket = 0;
     pg_search_stats sst{};
@@ -189,6 +193,7 @@ struct pg_job {
     pg_job_params prm{};
     std::shared_ptr<pg::Tables> T;
     uint32_t L = 0, sly = 0, W = 0, cap = 0;
+    uint32_t tcL = 0;  // operand words of the tensor-core search, 0 = not used
     uint32_t *d_wheel = nullptr;
     // jobs built without waiting on the device (PG_JOB_NO_GRAPH): the wheel
     // and the walk table are in place once this event completes

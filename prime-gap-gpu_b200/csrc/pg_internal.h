@@ -19,6 +19,9 @@ constexpr uint32_t TRIAL_PRIMES = 256;  // odd primes tried on positions past sl
 // next window's kernels can start on them.
 constexpr int PERSIST_THREADS = 32;
 
+// Words of a window's mu = floor(2^u / K) for the tensor-core search.
+constexpr int TC_MU_WORDS = 48;
+
 // One window of a search launch: the constants of the job it belongs to.  A
 // launch may carry windows of several jobs that share an operand layout; side
 // s (m index s >> 1) belongs to window wid[s >> 1], or window 0 when wid is
@@ -32,6 +35,11 @@ struct WinInfo {
     uint32_t confirm_rounds;           // record confirmation: total bases (< 2 = off)
     double k_log;                      // log(K), as the merit's denominator uses it
     double confirm_merit;              // m whose merit exceeds this get both primes confirmed
+    // tensor-core search (pg_tc.cuh): mu and the first byte column of the
+    // product with it that is computed
+    uint32_t mu[TC_MU_WORDS];
+    int32_t mu_off;
+    uint32_t side0, nsides;            // the window's sides in the launch
 };
 
 // A gap is confirmed when its approximate merit on the device exceeds
@@ -72,6 +80,13 @@ struct SearchArgs {
     // nothing, and a relaunch with the same arguments resumes at the queue head
     const volatile uint32_t *stop;  // NULL = never stop
     uint32_t *stopped;
+    // tensor-core search: a queue per window, since a CTA's candidates share
+    // their K
+    unsigned long long *win_next;      // [n_win] queue heads
+    uint32_t n_win;
+    uint32_t *rounds;                  // [2] rounds of tests started, and ended, by the launch's CTAs
+    uint32_t settle;                   // longest wait for the others' rounds, in 1/64 of the CTA's own
+    uint32_t *failed;                  // set when a matrix instruction did not complete
 };
 
 // Device scalars of one window slot.
@@ -86,6 +101,8 @@ struct Scalars {
     uint32_t unresolved;
     uint32_t active_warps;
     uint32_t stopped;  // the search left items queued (preempted)
+    uint32_t failed;   // the search gave up waiting for a matrix instruction
+    uint32_t rounds[2];
 };
 
 // Arguments of the sieve kernels for one window.
@@ -198,6 +215,11 @@ cudaError_t launch_imad_peak(int grid, uint32_t iters, uint32_t *sink, cudaStrea
 // records the calling thread's pg_last_error() text (pg_api.cu)
 void set_error(const char *msg);
 int search_grid(uint32_t L, int device);
+// Operand words of the tensor-core search for candidates m*K + X, m <= max_m,
+// |X| <= max_x, K of kbits bits with log2 K = k_log2; 0 where it does not apply.
+uint32_t pick_tc(uint32_t kbits, double k_log2, uint64_t max_m, uint64_t max_x);
+int tc_blocks_per_sm(uint32_t tcL);  // CTAs an SM holds
+cudaError_t launch_search_tc(uint32_t tcL, const SearchArgs &a, int grid, cudaStream_t st);
 bool supported_limbs(uint32_t L);
 uint32_t pick_limbs(uint32_t words);  // layout for operands of `words` words, 0 if none
 // layout for operands of `bits` bits: tpi 0 = automatic, 1 = one thread per

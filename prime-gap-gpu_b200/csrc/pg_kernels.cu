@@ -1010,6 +1010,8 @@ __global__ void k_init_search(uint32_t S, uint32_t *found_k, uint32_t *k_start, 
         sc->unresolved = S;
         sc->active_warps = warps;
         sc->stopped = 0;
+        sc->failed = 0;
+        sc->rounds[0] = sc->rounds[1] = 0;
     }
 }
 

@@ -251,11 +251,12 @@ extern "C" int pg_prp_batch_device(pg_ctx *c, const uint32_t *d_limbs, uint32_t 
     if (!d_limbs || !d_passed) return fail(PG_ERR_ARG, "pg_prp_batch_device: NULL buffer");
     if (words == 0 || words > PG_MAX_WORDS) return fail(PG_ERR_ARG, "pg_prp_batch_device: words=%u", words);
     if (rounds < 1 || rounds > 16) return fail(PG_ERR_ARG, "pg_prp_batch_device: rounds=%u (1..16)", rounds);
-    const uint32_t L = pick_limbs(words);
+    bool side_by_side = false;
+    const uint32_t L = pick_batch(words, n, rounds, &side_by_side);
     if (!L) return fail(PG_ERR_UNSUPPORTED, "pg_prp_batch_device: %u words above the compiled limit", words);
     cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
     PG_CUDA(cudaSetDevice(c->device));
-    PG_CUDA(launch_prp_batch(L, d_limbs, words, n, rounds, d_passed, st));
+    PG_CUDA(launch_prp_batch(L, d_limbs, words, n, rounds, d_passed, side_by_side, st));
     return PG_OK;
 }
 

@@ -56,17 +56,46 @@ uint32_t pick_layout(uint32_t bits, uint32_t tpi) {
 
 uint32_t pick_limbs(uint32_t words) { return pick_layout(32 * words, 0); }
 
+// A batch that does not fill the device takes the time of its longest chain:
+// the bases of a number one after the other, and the words of a squaring.
+// Bases run side by side while 16 lanes (or groups) per number still finish in
+// the time of one test: up to 16 384 tests of one thread each (22 words:
+// 2.05 ms for 16 and for 16 384 tests), or 18 944 lanes in groups (one warp per
+// SM quarter).  Few tests of more than 16 words take a group of lanes per
+// number; the layouts were timed against one thread per number:
+//   22 words 8 x 3: 1.66, 1.87, 2.53 ms at 2 048, 4 096, 8 192 tests (2.05 at each)
+//   32 words 16 x 3: 3.58, 4.19, 6.27 ms at 512, 2 048, 4 096 (5.8)
+//   40 words 16 x 3: 4.37, 5.13, 7.72 ms at 512, 2 048, 4 096 (10.8)
+//   48 words 8 x 8: 8.08, 10.8, 20.1 ms at 2 048, 4 096, 8 192 (18.7)
+// (16 words: 0.85 ms on one thread, 1.27 in groups).
+uint32_t pick_batch(uint32_t words, uint32_t n, uint32_t rounds, bool *side_by_side) {
+    const uint32_t L = pick_limbs(words);
+    *side_by_side = false;
+    if (!L) return 0;
+    if (L >> 16) {
+        *side_by_side = rounds > 1 && (uint64_t)n * 16 * (L >> 16) <= 18944;
+        return L;
+    }
+    *side_by_side = rounds > 1 && n <= 1024;
+    const uint32_t tests = *side_by_side ? 16 * n : n;
+    if (words > 16 && words <= 23 && tests <= 4096) return PG_LAYOUT_GROUP(8, 24);
+    if (words > 23 && words <= 47 && tests <= 64 * words) return PG_LAYOUT_GROUP(16, 48);
+    if (words == 48 && tests <= 4096) return PG_LAYOUT_GROUP(8, 64);
+    return L;
+}
+
 uint32_t layout_words(uint32_t layout) { return layout & 0xffffu; }
 
 cudaError_t launch_prp_batch(uint32_t L, const uint32_t *cand, uint32_t words, uint32_t n, uint32_t rounds,
-                             int32_t *out, cudaStream_t st) {
+                             int32_t *out, bool side_by_side, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
 #define PG_CASE(nl) \
-    if (L == nl) return launch_prp_batch_t<nl>(cand, words, n, rounds, out, st);
+    if (L == nl) return launch_prp_batch_t<nl>(cand, words, n, rounds, out, side_by_side, st);
     PG_LIMB_LIST(PG_CASE)
 #undef PG_CASE
 #define PG_GCASE(t, lt) \
-    if (L == PG_LAYOUT_GROUP(t, (t) * (lt))) return glaunch_prp_batch<t, lt>(cand, words, n, rounds, out, st);
+    if (L == PG_LAYOUT_GROUP(t, (t) * (lt)))            \
+        return glaunch_prp_batch<t, lt>(cand, words, n, rounds, out, side_by_side, st);
     PG_GROUP_LIST(PG_GCASE)
 #undef PG_GCASE
     return cudaErrorInvalidValue;

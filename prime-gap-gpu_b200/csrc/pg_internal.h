@@ -189,7 +189,7 @@ cudaError_t launch_walk_consts(const void *p, const void *c, const void *ci, boo
                                uint64_t count, uint32_t W, WalkC *out, cudaStream_t st);
 cudaError_t launch_sieve_small(const SieveArgs &a, bool compact, cudaStream_t st);
 cudaError_t launch_prp_batch(uint32_t L, const uint32_t *cand, uint32_t words, uint32_t n, uint32_t rounds,
-                             int32_t *out, cudaStream_t st);
+                             int32_t *out, bool side_by_side, cudaStream_t st);
 cudaError_t launch_search_persistent(uint32_t L, const SearchArgs &a, int grid, cudaStream_t st);
 cudaError_t launch_search_plain(uint32_t L, const SearchArgs &a, uint32_t *k_next, cudaStream_t st);
 cudaError_t launch_compact_active(const uint32_t *act_in, uint32_t n_in, const uint32_t *found_k,
@@ -222,6 +222,9 @@ int tc_blocks_per_sm(uint32_t tcL);  // CTAs an SM holds
 cudaError_t launch_search_tc(uint32_t tcL, const SearchArgs &a, int grid, cudaStream_t st);
 bool supported_limbs(uint32_t L);
 uint32_t pick_limbs(uint32_t words);  // layout for operands of `words` words, 0 if none
+// layout of a batch of n such operands tested with `rounds` bases, and whether
+// the bases of a number run side by side
+uint32_t pick_batch(uint32_t words, uint32_t n, uint32_t rounds, bool *side_by_side);
 // layout for operands of `bits` bits: tpi 0 = automatic, 1 = one thread per
 // number, T = groups of T lanes; 0 if none is compiled
 uint32_t pick_layout(uint32_t bits, uint32_t tpi);

@@ -383,6 +383,12 @@ __device__ __forceinline__ bool tiny_pass(const uint32_t (&n)[L], uint32_t base)
     return hi == 0 && n[0] - 1 <= base;
 }
 
+// base r of the strong test, r < 16
+__device__ __forceinline__ uint32_t prp_base(int r) {
+    const uint32_t bases[16] = {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53};
+    return bases[r & 15];
+}
+
 // number of bases (2, 3, 5, ...) passed before the first failure
 template <int L>
 __device__ __forceinline__ int prp_rounds(const uint32_t (&n)[L], int rounds) {

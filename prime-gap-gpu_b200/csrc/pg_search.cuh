@@ -36,6 +36,30 @@ __global__ void __launch_bounds__(128) k_prp_batch(const uint32_t *__restrict__ 
     out[i] = prp_rounds<L>(x, (int)rounds);
 }
 
+// The bases of one number side by side, 16 lanes a number: for batches so
+// small that the bases in turn would leave the device idle (12 numbers of 22
+// words, 16 bases: 48 ms in turn, the time of one test side by side).
+template <int L>
+__global__ void __launch_bounds__(128) k_prp_bases(const uint32_t *__restrict__ cand, uint32_t words, uint32_t n,
+                                                   uint32_t rounds, int32_t *__restrict__ out) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> 4, r = t & 15;
+    bool fail = false;
+    if (i < n && r < rounds) {
+        uint32_t x[L];
+        uint32_t hi = 0;
+#pragma unroll
+        for (int k = 0; k < L; k++) x[k] = ((uint32_t)k < words) ? cand[(size_t)i * words + k] : 0u;
+#pragma unroll
+        for (int k = 1; k < L; k++) hi |= x[k];
+        if ((x[0] & 1u) == 0 || (hi == 0 && x[0] < 3))
+            fail = true;
+        else
+            fail = !tiny_pass<L>(x, prp_base(r)) && !strong_prp<L>(x, prp_base(r));
+    }
+    const unsigned bad = (__ballot_sync(0xffffffffu, fail) >> (threadIdx.x & 16)) & 0xffffu;
+    if (i < n && r == 0) out[i] = bad ? __ffs(bad) - 1 : (int)rounds;
+}
+
 // ------------------------------------------------------------ search core
 
 // the window of side s
@@ -320,7 +344,11 @@ __global__ void __launch_bounds__(128) k_confirm(const __grid_constant__ SearchA
 
 template <int L>
 cudaError_t launch_prp_batch_t(const uint32_t *cand, uint32_t words, uint32_t n, uint32_t rounds, int32_t *out,
-                               cudaStream_t st) {
+                               bool side_by_side, cudaStream_t st) {
+    if (side_by_side) {
+        k_prp_bases<L><<<(n + 7) / 8, 128, 0, st>>>(cand, words, n, rounds, out);
+        return cudaGetLastError();
+    }
     const uint32_t threads = 128, blocks = (n + threads - 1) / threads;
     k_prp_batch<L><<<blocks, threads, 0, st>>>(cand, words, n, rounds, out);
     return cudaGetLastError();
@@ -365,7 +393,7 @@ cudaError_t launch_confirm_t(const SearchArgs &a, uint32_t *gaps, uint32_t *conf
 
 #define PG_DECLARE_LIMBS(L)                                                                                       \
     extern template cudaError_t launch_prp_batch_t<L>(const uint32_t *, uint32_t, uint32_t, uint32_t, int32_t *,  \
-                                                      cudaStream_t);                                              \
+                                                      bool, cudaStream_t);                                        \
     extern template int search_occupancy_t<L>();                                                                  \
     extern template cudaError_t launch_search_persistent_t<L>(const SearchArgs &, int, cudaStream_t);            \
     extern template cudaError_t launch_search_plain_t<L>(const SearchArgs &, uint32_t *, cudaStream_t);          \
@@ -375,7 +403,7 @@ cudaError_t launch_confirm_t(const SearchArgs &a, uint32_t *gaps, uint32_t *conf
                                                     uint32_t *, unsigned long long *, uint32_t *, cudaStream_t);
 
 #define PG_INSTANTIATE_LIMBS(L)                                                                                   \
-    template cudaError_t launch_prp_batch_t<L>(const uint32_t *, uint32_t, uint32_t, uint32_t, int32_t *,         \
+    template cudaError_t launch_prp_batch_t<L>(const uint32_t *, uint32_t, uint32_t, uint32_t, int32_t *, bool,   \
                                                cudaStream_t);                                                     \
     template int search_occupancy_t<L>();                                                                         \
     template cudaError_t launch_search_persistent_t<L>(const SearchArgs &, int, cudaStream_t);                   \

@@ -1,0 +1,37 @@
+"""Small PRP batches: bases side by side and lanes per number, at the sizes where pick_batch changes layout."""
+from __future__ import annotations
+
+import random
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+PSEUDO = [2047, 3277, 4033, 4681, 8321, 15841, 29341, 3215031751, 3474749660383, 341550071728321]
+
+
+def _mix(rng, bits, n):
+    """Primes, odd composites, pseudoprimes to the first bases, tiny, even and zero values, shuffled."""
+    import sympy
+    if bits < 800:
+        p = int(sympy.nextprime(rng.getrandbits(bits - 1) | (1 << (bits - 2))))
+    else:
+        p = 2 ** max(e for e in (607, 1279, 2203, 4253) if e <= bits) - 1
+    q = int(sympy.nextprime(rng.getrandbits(min(bits // 2, 400) - 1)))
+    fixed = [p, q, q * q, p - 2, 0, 1, 2, 3, 5, 7, 9, 47, 53, 54, 55, 2 ** 61 - 1] + PSEUDO
+    nums = [fixed[i % len(fixed)] if i % 3 == 0 else rng.getrandbits(bits) | 1 for i in range(n)]
+    rng.shuffle(nums)
+    nums[0] = (1 << bits) - 1 if n > 1 else p  # the batch's width
+    return nums
+
+
+@pytest.mark.parametrize("words,n,rounds", [
+    (1, 3, 16), (6, 40, 2), (16, 20, 16), (17, 1, 16), (22, 12, 16), (23, 9, 5), (23, 256, 2), (23, 257, 2),
+    (24, 7, 16), (24, 97, 2), (32, 128, 3), (32, 129, 3), (47, 30, 16), (48, 10, 16), (48, 257, 2), (22, 1024, 2),
+    (22, 1025, 2), (60, 148, 2), (60, 149, 2), (136, 6, 2), (22, 4096, 1), (22, 4097, 1), (28, 1793, 1)])
+def test_matches_the_oracle(ctx, oracle, words, n, rounds):
+    rng = random.Random(words * 1000 + n)
+    nums = _mix(rng, 32 * words, n)
+    got = ctx.prp(nums, rounds=rounds)
+    cut = range(n) if n <= 300 else sorted(rng.sample(range(n), 300))
+    assert [int(got[i]) for i in cut] == [oracle.prp(nums[i], rounds) for i in cut]

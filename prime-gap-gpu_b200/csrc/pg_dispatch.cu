@@ -149,6 +149,7 @@ uint32_t pick_tc(uint32_t kbits, double k_log2, uint64_t max_m, uint64_t max_x) 
 #undef PG_TCASE
     if (!best) return 0;
     if (n_log2 + m_log2 + 2.4 > 32.0 * (best + 1)) return 0;
+    if (kbits < 32 * (best - 4) + 25) return 0;  // mu no longer than its column offset + 1 (tc_mma)
     if ((double)kbits - 1 < 32.0 * (best - 4) + x_log2 + 8) return 0;
     return best;
 }

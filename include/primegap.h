@@ -244,8 +244,9 @@ int pg_next_prime_noalloc(const uint32_t *d_numbers, uint32_t n, uint32_t words,
  * would remain busy, handing their SMs to the next window (for callers that
  * keep another window submitted; a lone window finishes later with it);
  * D = (flags >> 8) & 0xff, 0 = 4.  PG_SUBMIT_WARPS_PER_SM(w) caps the PRP
- * kernel at w resident warps per SM (0 = as many as fit), leaving room for
- * the next window's kernels to run beside it.  pg_search() is submit + wait. */
+ * kernel at w resident warps per SM (0 = as many as fit; rounded up to whole
+ * thread blocks of 4 warps where the search runs on the tensor cores), leaving
+ * room for the next window's kernels to run beside it.  pg_search() is submit + wait. */
 #define PG_SEARCH_SLOTS 2
 #define PG_SUBMIT_DRAIN 0x1u
 #define PG_SUBMIT_DRAIN_LANES(d) (((uint32_t)(d) & 0xffu) << 8)

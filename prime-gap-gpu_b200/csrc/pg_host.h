@@ -132,6 +132,7 @@ struct Slot {
     uint32_t fin_round = 0, fin_ext = 0;
     int grid = 0, tc_grid = 0;
     uint32_t tc_settle = 0;  // SearchArgs::settle
+    bool shared = false;     // other launches run beside this one
     bool busy = false;
     uint64_t ticket = 0;
     pg_search_stats sst{};

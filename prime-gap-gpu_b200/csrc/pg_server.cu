@@ -532,6 +532,11 @@ struct pg_server {
                 if (!fill(ss)) break;
                 ss.seq = ++launch_seq;
                 ss.t_run = now();
+                ss.s.shared = running() > 0;
+                for (uint64_t id : order) {
+                    const Request &r = reqs.at(id);
+                    ss.s.shared |= r.state == St::ADMITTED && r.next_m < r.m_end;
+                }
                 int rc = slot_enqueue(ss.s, PG_SEARCH_PERSISTENT, PG_SUBMIT_WARPS_PER_SM(prm.warps_per_sm), false);
                 if (rc) {
                     fail_launch(lk, ss, rc, pg_last_error());

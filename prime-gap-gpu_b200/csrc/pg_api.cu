@@ -308,7 +308,7 @@ static int dalloc(uint64_t &acct, T **p, size_t count) {
 
 pg::Tables::~Tables() {
     cudaSetDevice(device);
-    void *ptrs[] = {d_sq, d_sr, d_sbar, d_tq, d_lp, d_lc, d_lcinv};
+    void *ptrs[] = {d_sq, d_sr, d_sbar, d_tq, d_lp, d_lc, d_lcinv, d_lat};
     for (void *p : ptrs) cudaFree(p);
 }
 
@@ -329,7 +329,7 @@ uint64_t pg::tables_bytes_estimate(const pg_job_params &p) {
     return (uint64_t)(3.0 * esz * pi_hi + 16.0 * q1 + (1u << 20));
 }
 
-static int tables_build(pg::Tables &T, const pg_job_params &p, cudaStream_t st) {
+static int tables_build(pg::Tables &T, const pg_job_params &p, uint64_t lat_bytes, cudaStream_t st) {
     // ---- K = P#/d
     std::vector<uint32_t> upto_p = host_primes(p.p);
     T.K.assign(1, 1);
@@ -471,13 +471,21 @@ static int tables_build(pg::Tables &T, const pg_job_params &p, cudaStream_t st) 
             cudaFree(oci);
             cudaFree(dep);
         }
+        if (e == cudaSuccess && acc && acc <= lat_bytes / sizeof(LatC)) {
+            uint64_t extra = 0;
+            if (!dalloc(extra, &T.d_lat, acc)) {
+                e = launch_lattices(T.d_lp, T.d_lc, T.d_lcinv, T.wide, acc, T.d_lat, st);
+                T.bytes += extra;
+            }
+            g_last_error.clear();
+        }
         free_scratch();
         if (e != cudaSuccess) return fail(PG_ERR_CUDA, "prime tables: %s", cudaGetErrorString(e));
     }
     return PG_OK;
 }
 
-int pg::tables_get(pg_ctx *c, const pg_job_params &p, std::shared_ptr<Tables> &out) {
+int pg::tables_get(pg_ctx *c, const pg_job_params &p, std::shared_ptr<Tables> &out, uint64_t lat_bytes) {
     const uint32_t q1 = small_bound(p);
     std::lock_guard<std::mutex> lock(c->tables_mu);
     auto &v = c->tables;
@@ -496,7 +504,7 @@ int pg::tables_get(pg_ctx *c, const pg_job_params &p, std::shared_ptr<Tables> &o
     t->d = p.d;
     t->max_prime = p.max_prime;
     t->q1 = q1;
-    int rc = tables_build(*t, p, c->stream);
+    int rc = tables_build(*t, p, lat_bytes, c->stream);
     if (rc) return rc;  // t frees what it holds
     t->setup_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     v.push_back(t);
@@ -679,6 +687,14 @@ static uint64_t seg_bands(const pg_job *j, uint64_t split, uint64_t nodd, SegBan
     return hi;
 }
 
+// First prime-table index sieved by the primes' lattices: those expecting at
+// most LAT_HITS hits in the window.
+static uint64_t lattice_first(const pg_job *j, uint64_t m0, uint64_t nodd) {
+    const pg::Tables &T = *j->T;
+    if (!T.d_lat || m0 >= (1ull << 30) || nodd >= (1ull << 30)) return T.np;
+    return table_index_at(T, (double)nodd * (2.0 * j->sly + 1) / LAT_HITS);
+}
+
 // sieve of one window of the slot into its rows of lists (compact) or into
 // the bitmap rows (the slot's first window only)
 static int run_sieve(Slot &s, const WinPart &w, bool compact) {
@@ -705,8 +721,10 @@ static int run_sieve(Slot &s, const WinPart &w, bool compact) {
     SegBand bands[MAX_SEG_BANDS];
     int nb = 0;
     const uint64_t search_first = seg_bands(j, split, w.nodd, bands, &nb);
-    PG_CUDA(launch_sieve_large(la, T.wide, split, bands, nb, search_first, s.st));
-    s.sst.kernel_launches += (split > 0) + (nb > 0) + (search_first < T.np);
+    const uint64_t lat_first = std::max(search_first, lattice_first(j, w.m0, w.nodd));
+    la.lat = lat_first < T.np ? T.d_lat : nullptr;
+    PG_CUDA(launch_sieve_large(la, T.wide, split, bands, nb, search_first, lat_first, s.st));
+    s.sst.kernel_launches += (split > 0) + (nb > 0) + (search_first < lat_first) + (lat_first < T.np);
     SieveArgs sa{};
     sa.sly = j->sly;
     sa.words = j->W;
@@ -1180,11 +1198,15 @@ static int job_build(pg_job *j) {
     if (2 * j->nm_cap >= 0xffffffffull) return fail(PG_ERR_UNSUPPORTED, "max_m_inc too large");
     // ---- walk steps of the large primes below 2^32 for this job's window width
     // (with PG_JOB_COMPACT_WALK only of those expecting >= SEG_HITS hits in the
-    // largest window, which the segmented kernel needs)
+    // largest window, which the segmented kernel needs; the lattices find the
+    // hits of those expecting at most LAT_HITS)
     if (T.np && !(p.flags & PG_JOB_LARGE_STEP)) {
         const uint64_t first = table_index_at(T, 2.0 * j->sly + 2);
-        double pmax = (p.flags & PG_JOB_COMPACT_WALK) ? (double)j->nodd_cap * (2.0 * j->sly + 1) / SEG_HITS
-                                                      : 4294967296.0;
+        double pmax = 4294967296.0;
+        if (p.flags & PG_JOB_COMPACT_WALK)
+            pmax = (double)j->nodd_cap * (2.0 * j->sly + 1) / SEG_HITS;
+        else if (T.d_lat && p.max_m < (1ull << 30))
+            pmax = (double)j->nodd_cap * (2.0 * j->sly + 1) / LAT_HITS;
         // table_index_at keeps the whole segment holding pmax: with primes above
         // 2^32 in the table, stop a segment early so every kept prime is below 2^32
         if (T.wide) pmax = std::min(pmax, 4294967296.0 - (double)T.seg_span);

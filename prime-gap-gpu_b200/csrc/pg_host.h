@@ -58,6 +58,7 @@ struct Tables {
     uint32_t *d_tq = nullptr;   // trial primes 3, 5, 7, ...
     std::vector<uint32_t> tr;   // their residues (-(K mod q)/2) mod q
     void *d_lp = nullptr, *d_lc = nullptr, *d_lcinv = nullptr;
+    LatC *d_lat = nullptr;  // reduced lattices of the primes; NULL = not kept (memory)
     uint64_t np = 0;
     bool wide = false;
     // prime-table index of each sieve segment (segment s starts at value seg_v0 + s * seg_span)
@@ -69,9 +70,11 @@ struct Tables {
 };
 
 // The tables of (p, d, max_prime, small_limit) on ctx: a live copy shared with
-// other jobs, else a new build.
-int tables_get(pg_ctx *c, const pg_job_params &p, std::shared_ptr<Tables> &out);
-// Device bytes a build of those tables would take (an upper estimate).
+// other jobs, else a new build.  The lattices (16 B a prime) are kept where
+// they take no more than lat_bytes and the device has room.
+int tables_get(pg_ctx *c, const pg_job_params &p, std::shared_ptr<Tables> &out, uint64_t lat_bytes = ~0ull);
+// Device bytes a build of those tables would take without the lattices (an
+// upper estimate).
 uint64_t tables_bytes_estimate(const pg_job_params &p);
 
 // One window of a slot.

@@ -130,6 +130,7 @@ struct SieveArgs {
 };
 
 struct WalkC;
+struct LatC;
 
 struct LargeArgs {
     uint32_t sly;
@@ -145,6 +146,7 @@ struct LargeArgs {
     const uint32_t *wheel;  // [words] positions composite in every row (Y = 0, q | Y for q | K)
     const struct WalkC *walk;  // walk steps of the primes [walk_first, walk_end), NULL = none
     uint64_t walk_first, walk_end;
+    const struct LatC *lat;    // reduced lattice of every prime, NULL = none (m0 < 2^30 and nodd < 2^30 only)
 };
 
 // The three-distance walk of one prime below 2^32: the step counts sa (the
@@ -155,6 +157,21 @@ struct LargeArgs {
 struct WalkC {
     uint32_t sa, sb;
 };
+
+// The lattice {(x, S): A*x + S = 0 mod p} of one prime (A = -K), as the hits of
+// a window enumerate it: with the steps (sa, alpha), (sb, -beta) of WalkC for
+// the width LAT_W, its points are x = Q*M - t*inc, S = t*dec + Q*w over the
+// integers t, Q, where
+//   alpha >= beta: M = sb, inc = sa mod sb, w = beta, dec = alpha + (sa / sb) beta
+//   else:          M = sa, inc = -sb mod sa, w = -alpha, dec = beta + ceil(sb / sa) alpha
+// They depend on p and K mod p only.  M = 0: kept out of the enumeration
+// (p too small for the width, or a value out of range).
+struct LatC {
+    uint32_t M, inc, dec;
+    int32_t w;
+};
+constexpr uint32_t LAT_W = 1u << 13;
+constexpr double LAT_HITS = 1.0;
 
 // Primes of the large-prime table processed by the segmented kernel in one
 // launch: [first, first + count), each split into nseg segments of seg_len
@@ -181,12 +198,16 @@ cudaError_t launch_prime_reorder(uint64_t np, uint32_t nseg, const uint64_t *seg
                                  cudaStream_t st);
 // Large-prime sieve of one window: primes [0, split) step every Y; the bands
 // run the segmented walk (the walk steps of a.walk); primes [search_first,
-// np) one thread each (modular search for the first hit, then the walk).
+// lat_first) one thread each (modular search for the first hit, then the
+// walk); primes [lat_first, np) one thread each by their lattices (a.lat).
 cudaError_t launch_sieve_large(const LargeArgs &a, bool wide, uint64_t split, const SegBand *bands, int nbands,
-                               uint64_t search_first, cudaStream_t st);
+                               uint64_t search_first, uint64_t lat_first, cudaStream_t st);
 // walk constants of the primes [first, first + count) (all < 2^32) for width W
 cudaError_t launch_walk_consts(const void *p, const void *c, const void *ci, bool wide, uint64_t first,
                                uint64_t count, uint32_t W, WalkC *out, cudaStream_t st);
+// reduced lattices of the table's primes
+cudaError_t launch_lattices(const void *p, const void *c, const void *ci, bool wide, uint64_t np, LatC *out,
+                            cudaStream_t st);
 cudaError_t launch_sieve_small(const SieveArgs &a, bool compact, cudaStream_t st);
 cudaError_t launch_prp_batch(uint32_t L, const uint32_t *cand, uint32_t words, uint32_t n, uint32_t rounds,
                              int32_t *out, bool side_by_side, cudaStream_t st);

@@ -268,8 +268,11 @@ struct pg_server {
                     continue;  // wait for memory
                 }
                 std::shared_ptr<Tables> T;
+                // the lattices may take a quarter of what the budget leaves, so
+                // they never keep another table set out for long
+                const uint64_t spare = (prm.hbm_budget - resident() - need) / 4;
                 lk.unlock();
-                int rc = tables_get(ctx, tp, T);
+                int rc = tables_get(ctx, tp, T, spare);
                 std::string err = rc ? pg_last_error() : "";
                 lk.lock();
                 if (rc) {

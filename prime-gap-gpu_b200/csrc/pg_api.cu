@@ -833,12 +833,12 @@ static int enqueue_windows(Slot &s, int form, uint32_t flags) {
         }
         // a draining launch counts warps that leave one by one: the one-warp kernel
         s.search_tc = s.tcL && !a.drain_lanes;
+        a.settle = s.settle;
+        a.rounds = s.d_sc->rounds;
         if (s.search_tc) {
             a.win_next = s.d_wnext;
             a.n_win = (uint32_t)s.parts.size();
             a.failed = &s.d_sc->failed;
-            a.settle = s.tc_settle;
-            a.rounds = s.d_sc->rounds;
             PG_CUDA(cudaMemsetAsync(s.d_wnext, 0, s.parts.size() * 8, s.st));
         }
         s.search = a;
@@ -909,22 +909,27 @@ int pg::slot_resume(Slot &s) {
     return enqueue_finalize(s, a, S);
 }
 
-// CTAs of the tensor-core search for the slot's sides.  Every CTA tests 128
-// candidates at a time, the nearest of the sides still open, and c of them on
-// an SM take about 1 + 0.43 (c - 1) times as long per round as one (L = 23:
-// 3 800, 5 400, 6 900, 8 900 cycles a step at c = 1 .. 4).  A side takes
-// 1 / p tests on average, p = e^gamma ln(max_prime) / ln N, so a round of
-// `lanes` tests leaves a share exp(-p * lanes / open) of the open sides.  Many
-// sides want every CTA that fits; few sides want the shorter rounds, since
-// the deeper candidates of a fuller device are tested for nothing.  The CTAs
-// of a round end within a few per cent of each other, and those that end
-// first would refill with the next candidates of sides whose prime the others
-// are about to report, so with few rounds each CTA waits, at most an eighth of
-// its round, until the rounds begun before its own ended have ended too.  A
-// launch that shares the device takes all CTAs and never waits (15 mixed
-// requests on a server: 201 ms with the rule on every launch, 178 without).
-static int tc_ctas(Slot &s) {
-    const int sms = s.parts[0].job->ctx->sms, most = tc_blocks_per_sm(s.tcL);
+// Blocks per SM of a search over the slot's sides.  Every block tests `per`
+// candidates at a time, the nearest of the sides still open, and c blocks on an
+// SM take 1 + slope (c - step) / step times as long per round as `step` of
+// them (one per SM quarter).  A side takes 1 / p tests on average,
+// p = e^gamma ln(max_prime) / ln N, so a round of `lanes` tests leaves a share
+// exp(-p * lanes / open) of the open sides.  Many sides want every block that
+// fits; few sides want the shorter rounds, since the deeper candidates of a
+// fuller device are tested for nothing.  The blocks of a round end within a few
+// per cent of each other, and those that end first would refill with the next
+// candidates of sides whose prime the others are about to report, so with few
+// rounds each block waits, at most an eighth of its round, until the rounds
+// begun before its own ended have ended too.  A launch that shares the device
+// takes all blocks and never waits (15 mixed requests on a server: 201 ms with
+// the rule on every launch, 178 without).
+//   tensor-core kernel, per = 128, step 1, slope 0.43 (L = 23: 3 800, 5 400,
+//   6 900, 8 900 cycles a step at c = 1 .. 4): 345 m of P = 503 4.98 ms at
+//   c = 4, 3.2 with the rule; 1 000 m of P = 907 15.7 and 12.1 ms
+//   lane groups, per = 32 / T, step 4, slope 0.57 (8 x 17: 70, 112, 150 ms a
+//   test at c = 4, 8, 12)
+static int round_blocks(Slot &s, int most, int step, double slope, double per) {
+    const int sms = s.parts[0].job->ctx->sms;
     double tests = 0, sides = 0;
     for (const WinPart &w : s.parts) {
         const pg_job *j = w.job;
@@ -934,24 +939,24 @@ static int tc_ctas(Slot &s) {
     }
     const double per_side = tests / std::max(sides, 1.0);
     int best = most;
-    s.tc_settle = 0;
+    s.settle = 0;
     double best_t = 1e300;
-    for (int c = most; c >= 1; c--) {
-        const double lanes = (double)c * sms * 128;
+    for (int c = most; c >= step; c -= step) {
+        const double lanes = (double)c * sms * per;
         if (tests > 24 * lanes) break;  // throughput decides
         double open = sides, rounds = 0;
         while (open > 0.05 && rounds < 100) {
             open *= std::exp(-lanes / (open * per_side));
             rounds++;
         }
-        const double t = rounds * (1 + 0.43 * (c - 1));
+        const double t = rounds * (1 + slope * (c - step) / step);
         if (t < best_t) {
             best_t = t;
             best = c;
-            s.tc_settle = 8;
+            s.settle = 8;
         }
     }
-    return sms * best;
+    return best;
 }
 
 int pg::slot_enqueue(Slot &s, int form, uint32_t flags, bool graph) {
@@ -963,23 +968,21 @@ int pg::slot_enqueue(Slot &s, int form, uint32_t flags, bool graph) {
     s.grid = search_grid(s.L, s.parts[0].job->ctx->device);
     const uint32_t wps = (flags >> 16) & 0xffu;  // warps per SM cap
     if (wps) s.grid = std::min(s.grid, s.parts[0].job->ctx->sms * (int)wps * 32 / PERSIST_THREADS);
+    const int sms = s.parts[0].job->ctx->sms;
+    s.settle = 0;
     if (s.tcL) {
-        if (s.shared) {
-            s.tc_settle = 0;
-            s.tc_grid = s.parts[0].job->ctx->sms * tc_blocks_per_sm(s.tcL);
-        } else {
-            s.tc_grid = tc_ctas(s);
-        }
-        if (wps) {
+        const int most = tc_blocks_per_sm(s.tcL);
+        if (wps)
             // another launch runs beside this one: the cap in whole CTAs of 4
             // warps, and at most half of those that fit, so both find room
             // (P = 503, two windows of 200 000 m in flight at a cap of 6: 77.4 ms
             // a window at 1.5 CTAs per SM, 71.0 at 2; P = 907, where two fit:
             // 42.4 ms at 1, 47.0 at 2)
-            const int c = std::min(((int)wps + 3) / 4, (tc_blocks_per_sm(s.tcL) + 1) / 2);
-            s.tc_grid = std::min(s.tc_grid, s.parts[0].job->ctx->sms * c);
-            s.tc_settle = 0;
-        }
+            s.tc_grid = sms * std::min(((int)wps + 3) / 4, (most + 1) / 2);
+        else
+            s.tc_grid = sms * (s.shared ? most : round_blocks(s, most, 1, 0.43, 128));
+    } else if ((s.L >> 16) && !wps && !s.shared && form == PG_SEARCH_PERSISTENT && !(flags & PG_SUBMIT_DRAIN)) {
+        s.grid = sms * round_blocks(s, s.grid / sms, 4, 0.57, 32.0 / (s.L >> 16));
     }
     if (form == PG_SEARCH_PLAIN || !graph) return enqueue_windows(s, form, flags);
     // The persistent form's whole window (upload, sieves, search, finalize,
@@ -1062,7 +1065,11 @@ int pg::slot_finish(Slot &s, bool wait) {
         a.kspan = s.stride + ext_new;
         a.max_count = nullptr;
         PG_CUDA(cudaMemsetAsync(&s.d_sc->next_item, 0, 8, s.st));
-        PG_CUDA(launch_search_persistent(s.L, a, s.grid, s.st));
+        // a few sides: one warp per SM quarter (fuller SMs lengthen the test for
+        // deeper candidates of the same sides)
+        const int sms = s.parts[0].job->ctx->sms;
+        const int grid = n_redo <= 4u * sms ? std::min(s.grid, 4 * sms) : s.grid;
+        PG_CUDA(launch_search_persistent(s.L, a, grid, s.st));
         s.sst.kernel_launches++;
         s.sst.relaunches++;
         s.sst.extended_sides += n_redo;

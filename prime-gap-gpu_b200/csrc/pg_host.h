@@ -134,7 +134,7 @@ struct Slot {
     int fin_phase = 0;
     uint32_t fin_round = 0, fin_ext = 0;
     int grid = 0, tc_grid = 0;
-    uint32_t tc_settle = 0;  // SearchArgs::settle
+    uint32_t settle = 0;     // SearchArgs::settle
     bool shared = false;     // other launches run beside this one
     bool busy = false;
     uint64_t ticket = 0;

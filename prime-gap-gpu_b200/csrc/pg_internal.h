@@ -80,12 +80,14 @@ struct SearchArgs {
     // nothing, and a relaunch with the same arguments resumes at the queue head
     const volatile uint32_t *stop;  // NULL = never stop
     uint32_t *stopped;
+    // launches of few rounds (tensor-core and lane-group kernels): a CTA whose
+    // round of tests ended waits for the rounds begun before that
+    uint32_t *rounds;                  // [2] rounds begun and ended by the launch's CTAs
+    uint32_t settle;                   // longest wait, in 1/64 of the CTA's own round; 0 = none
     // tensor-core search: a queue per window, since a CTA's candidates share
     // their K
     unsigned long long *win_next;      // [n_win] queue heads
     uint32_t n_win;
-    uint32_t *rounds;                  // [2] rounds of tests started, and ended, by the launch's CTAs
-    uint32_t settle;                   // longest wait for the others' rounds, in 1/64 of the CTA's own
     uint32_t *failed;                  // set when a matrix instruction did not complete
 };
 

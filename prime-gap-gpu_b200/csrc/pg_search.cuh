@@ -119,6 +119,19 @@ __device__ __forceinline__ void stop_check(const SearchArgs &a, unsigned long lo
     }
 }
 
+// Called by one thread of a CTA when the CTA's round of tests, begun at clock
+// t_round, has ended and its results are written and fenced: waits, within the
+// limit, for the rounds that were begun before that.
+__device__ __forceinline__ void settle_round(const SearchArgs &a, long long t_round) {
+    const long long t0 = clock64(), limit = (t0 - t_round) * a.settle >> 6;
+    const uint32_t begun = *(volatile const uint32_t *)&a.rounds[0];
+    uint32_t ended = atomicAdd(&a.rounds[1], 1u) + 1;
+    while ((int32_t)(ended - begun) < 0 && clock64() - t0 < limit) {
+        __nanosleep(200);
+        ended = *(volatile const uint32_t *)&a.rounds[1];
+    }
+}
+
 // Resolves work item (side s, k-th candidate) to its position Y, or returns
 // false when the item needs no test: the side already has a probable prime
 // at a smaller k, the item lies past this launch's extension window, or an

@@ -161,6 +161,8 @@ __global__ void __launch_bounds__(PERSIST_THREADS) k_search_persistent_g(const _
             }
         }
         if (!__any_sync(FULL, have)) break;
+        const long long t_round = clock64();
+        if (a.settle && G.lane == 0) atomicAdd(&a.rounds[0], 1u);
         if (have) {
             uint32_t x[LT];
             gbuild_candidate<T, LT>(G, win_of(a, s).K, a.ms[s >> 1], Y, s & 1, x);
@@ -170,6 +172,11 @@ __global__ void __launch_bounds__(PERSIST_THREADS) k_search_persistent_g(const _
                 if (pr && atomicMin(&a.found_k[s], k) == NOT_FOUND && a.unresolved) atomicSub(a.unresolved, 1u);
             }
             have = false;
+        }
+        if (a.settle) {  // wait for the rounds under way (see round_blocks in pg_api.cu)
+            __threadfence();
+            __syncwarp();
+            if (G.lane == 0) settle_round(a, t_round);
         }
     }
     __syncwarp();

@@ -221,18 +221,10 @@ __global__ void __launch_bounds__(TC_ROWS, tc_min_blocks(L)) k_search_tc(const _
             ntests++;
             if (pr && atomicMin(&a.found_k[s], k) == NOT_FOUND && a.unresolved) atomicSub(a.unresolved, 1u);
         }
-        if (a.settle) {  // wait, within the limit, for the rounds under way (see tc_ctas in pg_api.cu)
+        if (a.settle) {  // wait, within the limit, for the rounds under way (see round_blocks in pg_api.cu)
             __threadfence();
             __syncthreads();
-            if (tid == 0) {
-                const long long t0 = clock64(), limit = (t0 - t_round) * a.settle >> 6;
-                const uint32_t begun = *(volatile const uint32_t *)&a.rounds[0];
-                uint32_t ended = atomicAdd(&a.rounds[1], 1u) + 1;
-                while ((int32_t)(ended - begun) < 0 && clock64() - t0 < limit) {
-                    __nanosleep(200);
-                    ended = *(volatile const uint32_t *)&a.rounds[1];
-                }
-            }
+            if (tid == 0) settle_round(a, t_round);
         }
     }
 #pragma unroll

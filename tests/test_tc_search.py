@@ -119,3 +119,13 @@ def test_short_sieve_and_extension(pg):
         a = job.search(1_000_000, 20_000)
         b = job.wait(job.submit(1_000_000, 20_000, flags=pg.PG_SUBMIT_DRAIN))
     assert np.array_equal(a.prev_gap, b.prev_gap) and np.array_equal(a.next_gap, b.next_gap)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m_inc", [2, 40, 400])
+def test_lane_groups_few_sides(pg, m_inc):
+    """Lane-group searches on grids of one warp per SM quarter and more, against every block with draining."""
+    with pg.Job(337, 2310, 5_000, 10_000_000, max_m_inc=m_inc, max_m=10_100_000, tpi=8) as job:
+        a = job.search(10_000_001, m_inc)
+        b = job.wait(job.submit(10_000_001, m_inc, flags=pg.PG_SUBMIT_DRAIN))
+    assert np.array_equal(a.prev_gap, b.prev_gap) and np.array_equal(a.next_gap, b.next_gap)

@@ -1106,8 +1106,26 @@ int pg::slot_finish(Slot &s, bool wait) {
 // ================================================================= jobs
 
 extern "C" uint64_t pg_count_m(uint64_t m_start, uint64_t m_inc, uint32_t d) {
-    uint64_t c = 0;
-    for (uint64_t m = m_start; m < m_start + m_inc; m++) c += gcd64(m, d) == 1;
+    const uint64_t end = m_start + m_inc;
+    if (end <= m_start) return 0;  // empty, or past 2^64
+    if (d == 0) return m_start <= 1 && end > 1;  // gcd(m, 0) = m
+    // inclusion and exclusion over the products of d's primes (at most 9)
+    uint64_t e[512], c = 0;
+    int n = 1;
+    e[0] = 1;
+    uint32_t r = d;
+    for (uint32_t q = 2; r > 1; q++) {
+        if ((uint64_t)q * q > r) q = r;
+        if (r % q) continue;
+        while (r % q == 0) r /= q;
+        for (int i = 0; i < n; i++) e[n + i] = e[i] * q;
+        n *= 2;
+    }
+    // e[i] has as many primes as i has bits; multiples of e in [m_start, end)
+    for (int i = 0; i < n; i++) {
+        const uint64_t k = (end - 1) / e[i] + 1 - (m_start ? (m_start - 1) / e[i] + 1 : 0);
+        c += __builtin_popcount((unsigned)i) & 1 ? 0 - k : k;
+    }
     return c;
 }
 

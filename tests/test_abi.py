@@ -39,6 +39,15 @@ def test_count_m_matches_oracle(pg, oracle, m_start, m_inc, d):
     assert pg.count_m(m_start, m_inc, d) == len(oracle.coprime_ms(m_start, m_inc, d))
 
 
+@pytest.mark.parametrize("d", [0, 1, 2, 3, 4, 12, 30, 2190, 49, 9973, 223_092_870, 4_294_967_291, 4_294_836_225])
+def test_count_m_edges(pg, d):
+    import math
+    for start, inc in [(0, 0), (0, 1), (0, 7), (1, 0), (1, 1), (5, 300), (9_970, 9), (2 ** 40 + 1, 200),
+                       (2 ** 64 - 300, 299), (2 ** 64 - 300, 300), (2 ** 64 - 5, 10)]:
+        end = (start + inc) % 2 ** 64
+        assert pg.count_m(start, inc, d) == sum(math.gcd(m, d) == 1 for m in range(start, end))
+
+
 def test_counts_of_the_benchmark_windows(pg):
     # coprime m of the four benchmark windows: 2,079 / 52,604 / 11,429 / 26,300
     assert pg.count_m(10_000_000, 10_000, 2310) == 2079

@@ -916,15 +916,18 @@ int pg::slot_resume(Slot &s) {
 // p = e^gamma ln(max_prime) / ln N, so a round of `lanes` tests leaves a share
 // exp(-p * lanes / open) of the open sides.  Many sides want every block that
 // fits; few sides want the shorter rounds, since the deeper candidates of a
-// fuller device are tested for nothing.  The blocks of a round end within a few
-// per cent of each other, and those that end first would refill with the next
-// candidates of sides whose prime the others are about to report, so with few
-// rounds each block waits, at most an eighth of its round, until the rounds
-// begun before its own ended have ended too.  A launch that shares the device
+// fuller device are tested for nothing.  The blocks that end a round first
+// would refill with the next candidates of sides whose prime the others are
+// about to report, so each block waits until the rounds begun before its own
+// ended have ended too, at most a quarter of its round (an eighth in searches
+// of more than 12 rounds, where the waits cost more than they save): 10 000 m
+// of P = 337 2.91 ms at an eighth, 2.58 at a quarter; 20 000 m of P = 907 74.2
+// without, 61.9 at either; 200 000 m of P = 503 69.1, 69.9 and 71.5.  A launch that shares the device
 // takes all blocks and never waits (15 mixed requests on a server: 201 ms with
 // the rule on every launch, 178 without).
-//   tensor-core kernel, per = 128, step 1, slope 0.43 (L = 23: 3 800, 5 400,
-//   6 900, 8 900 cycles a step at c = 1 .. 4): 345 m of P = 503 4.98 ms at
+//   tensor-core kernel, per = 128, step 1, slope 0.33 (L = 15: 2 520, 3 520,
+//   4 090, 5 000 cycles a step at c = 1 .. 4), 0.43 (L = 23: 3 800, 4 940, 7 020,
+//   8 910) or 0.37 (L = 40: 8 020, 11 030 at c = 1, 2): 345 m of P = 503 4.98 ms at
 //   c = 4, 3.2 with the rule; 1 000 m of P = 907 15.7 and 12.1 ms
 //   lane groups, per = 32 / T, step 4, slope 0.57 (8 x 17: 70, 112, 150 ms a
 //   test at c = 4, 8, 12)
@@ -953,7 +956,7 @@ static int round_blocks(Slot &s, int most, int step, double slope, double per) {
         if (t < best_t) {
             best_t = t;
             best = c;
-            s.settle = 8;
+            s.settle = rounds <= 12 ? 16 : 8;
         }
     }
     return best;
@@ -980,7 +983,7 @@ int pg::slot_enqueue(Slot &s, int form, uint32_t flags, bool graph) {
             // 42.4 ms at 1, 47.0 at 2)
             s.tc_grid = sms * std::min(((int)wps + 3) / 4, (most + 1) / 2);
         else
-            s.tc_grid = sms * (s.shared ? most : round_blocks(s, most, 1, 0.43, 128));
+            s.tc_grid = sms * (s.shared ? most : round_blocks(s, most, 1, s.tcL < 20 ? 0.33 : s.tcL < 30 ? 0.43 : 0.37, 128));
     } else if ((s.L >> 16) && !wps && !s.shared && form == PG_SEARCH_PERSISTENT && !(flags & PG_SUBMIT_DRAIN)) {
         s.grid = sms * round_blocks(s, s.grid / sms, 4, 0.57, 32.0 / (s.L >> 16));
     }

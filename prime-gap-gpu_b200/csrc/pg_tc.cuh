@@ -250,9 +250,10 @@ struct TcState {
 
 // One squaring of every row of the CTA (all 128 threads call it).  m < 2^30,
 // xabs < 2^24; ratio = -X * 2^(32 (NZ-TOP)) / n.  A wait that ran out clears
-// S.ok; the threads agree on it at the next barrier and all leave.
+// S.ok; the threads agree on it at the next barrier, and the call that holds
+// that barrier returns false in all of them.
 template <int L>
-__device__ __forceinline__ void tc_step(TcState &S, uint32_t (&y)[L], uint32_t m, uint32_t xabs, uint32_t xneg,
+__device__ __forceinline__ bool tc_step(TcState &S, uint32_t (&y)[L], uint32_t m, uint32_t xabs, uint32_t xneg,
                                         double ratio, uint32_t dbl) {
     using D = TcDim<L>;
     uint32_t T[2 * L];
@@ -261,7 +262,7 @@ __device__ __forceinline__ void tc_step(TcState &S, uint32_t (&y)[L], uint32_t m
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     S.ok = __syncthreads_and(S.ok);
-    if (!S.ok) return;
+    if (!S.ok) return false;
     if (S.lead) {
         tc_fence_after();
         tc_mma<D::N1, D::K1, false>(S.tmem, S.a, S.b1);
@@ -290,7 +291,7 @@ __device__ __forceinline__ void tc_step(TcState &S, uint32_t (&y)[L], uint32_t m
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     S.ok = __syncthreads_and(S.ok);
-    if (!S.ok) return;
+    if (!S.ok) return false;
     if (S.lead) {
         tc_fence_after();
         tc_mma<D::N2, D::K2, true>(S.tmem, S.a, S.b2);
@@ -318,6 +319,7 @@ __device__ __forceinline__ void tc_step(TcState &S, uint32_t (&y)[L], uint32_t m
     for (int k = 2; k < L; k++)
         y[k] = k + 1 < L ? addc_cc((uint32_t)v[k], (uint32_t)(v[k - 1] >> 32))
                          : addc((uint32_t)v[k], (uint32_t)(v[k - 1] >> 32));
+    return true;
 }
 
 // j = -X^-1 mod m (X = +-xabs); false when gcd(m, X) > 1

@@ -210,8 +210,7 @@ __global__ void __launch_bounds__(TC_ROWS, tc_min_blocks(L)) k_search_tc(const _
                 }
             }
             if (b == 0) break;
-            tc_step<L>(S, y, m, xabs, prev ? 0xffffffffu : 0u, ratio, (ew >> (b & 31)) & 1u);
-            if (!S.ok) break;
+            if (!tc_step<L>(S, y, m, xabs, prev ? 0xffffffffu : 0u, ratio, (ew >> (b & 31)) & 1u)) break;
         }
         if (!__syncthreads_and(S.ok)) {
             if (tid == 0) atomicExch(a.failed, 1u);

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(16 * T) k_prp_bases_g(const uint32_t *__restri
         const bool big = G.field(__ballot_sync(G.gmask, hi != 0)) != 0;
         const uint32_t n0 = __shfl_sync(G.gmask, x[0], G.gb), base = prp_base(r);
         bool fail = (n0 & 1u) == 0 || (!big && n0 < 3);
-        if (!fail && (big || n0 - 1 > base)) fail = !gstrong_prp<T, LT>(G, x, base);
+        if (!fail && (big || n0 - 1 > base)) fail = !gstrong_prp<T, LT, true>(G, x, base);
         if (fail && G.gl == 0) atomicOr(&s_bad, 1u << r);
     }
     __syncthreads();

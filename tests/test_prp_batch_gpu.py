@@ -35,3 +35,18 @@ def test_matches_the_oracle(ctx, oracle, words, n, rounds):
     got = ctx.prp(nums, rounds=rounds)
     cut = range(n) if n <= 300 else sorted(rng.sample(range(n), 300))
     assert [int(got[i]) for i in cut] == [oracle.prp(nums[i], rounds) for i in cut]
+
+
+@pytest.mark.parametrize("words", [64, 96])
+def test_bases_at_the_width_of_the_lanes(ctx, oracle, words):
+    """Operands with 7, 8 and 9 bits to spare in their lanes, and none: folded and multiplied bases side by side."""
+    bits = 32 * words
+    nums = []
+    for spare in (0, 7, 8, 9):
+        top = 1 << (bits - spare)
+        nums += [top - 1, (top >> 1) + 1, top - 2 ** (bits // 3) + 1]
+    for e in (1279, 2203):
+        if e <= bits:
+            nums += [2 ** e - 1, (2 ** e - 1) * ((1 << (bits - e - 8)) | 1)]
+    got = ctx.prp(nums, rounds=16)
+    assert [int(g) for g in got] == [oracle.prp(x, 16) for x in nums]

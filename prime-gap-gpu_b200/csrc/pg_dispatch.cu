@@ -67,6 +67,12 @@ uint32_t pick_limbs(uint32_t words) { return pick_layout(32 * words, 0); }
 //   32 words 16 x 3: 3.58, 4.19, 6.27 ms at 512, 2 048, 4 096 (5.8)
 //   40 words 16 x 3: 4.37, 5.13, 7.72 ms at 512, 2 048, 4 096 (10.8)
 //   48 words 8 x 8: 8.08, 10.8, 20.1 ms at 2 048, 4 096, 8 192 (18.7)
+// Longer operands are in groups already; 16 lanes instead of 8 halve a row's
+// products on a lane, for twice the warps:
+//   95 words 16 x 6: 19.2, 25.8, 36.3, 47.5 ms at 1 184, 2 368, 3 072, 4 096
+//            8 x 12: 27.5, 27.5, 39.7, 39.7
+//  135 words 16 x 9: 45.8, 66.9, 101.2 ms at 1 184, 2 368, 3 072
+//            8 x 17: 70.8, 70.8, 101.6
 // (16 words: 0.85 ms on one thread, 1.27 in groups).
 uint32_t pick_batch(uint32_t words, uint32_t n, uint32_t rounds, bool *side_by_side) {
     const uint32_t L = pick_limbs(words);
@@ -74,6 +80,9 @@ uint32_t pick_batch(uint32_t words, uint32_t n, uint32_t rounds, bool *side_by_s
     if (!L) return 0;
     if (L >> 16) {
         *side_by_side = rounds > 1 && (uint64_t)n * 16 * (L >> 16) <= 18944;
+        const uint32_t tests = *side_by_side ? 16 * n : n;
+        if (L == PG_LAYOUT_GROUP(8, 96) && tests <= 3072) return PG_LAYOUT_GROUP(16, 96);
+        if (L == PG_LAYOUT_GROUP(8, 136) && tests <= 2368) return PG_LAYOUT_GROUP(16, 144);
         return L;
     }
     *side_by_side = rounds > 1 && n <= 1024;

@@ -10,7 +10,7 @@
 #define PG_LIMB_LIST(X) X(4) X(8) X(12) X(15) X(16) X(20) X(22) X(23) X(24) X(28) X(32) X(36) X(40) X(44) X(48)
 
 #define PG_GROUP_LIST(X) \
-    X(8, 3) X(4, 6) X(4, 8) X(4, 10) X(4, 12) X(8, 8) X(8, 12) X(8, 17) X(8, 20) X(16, 2) X(16, 3) X(16, 9)
+    X(8, 3) X(4, 6) X(4, 8) X(4, 10) X(4, 12) X(8, 8) X(8, 12) X(8, 17) X(8, 20) X(16, 2) X(16, 3) X(16, 6) X(16, 9)
 
 // PG_TC_LIST: operand words of the searches that reduce on the tensor cores
 // (pg_tc_search.cuh); the next larger entry takes the sizes between.  Steps of

@@ -28,7 +28,9 @@ def _mix(rng, bits, n):
 @pytest.mark.parametrize("words,n,rounds", [
     (1, 3, 16), (6, 40, 2), (16, 20, 16), (17, 1, 16), (22, 12, 16), (23, 9, 5), (23, 256, 2), (23, 257, 2),
     (24, 7, 16), (24, 97, 2), (32, 128, 3), (32, 129, 3), (47, 30, 16), (48, 10, 16), (48, 257, 2), (22, 1024, 2),
-    (22, 1025, 2), (60, 148, 2), (60, 149, 2), (136, 6, 2), (22, 4096, 1), (22, 4097, 1), (28, 1793, 1)])
+    (22, 1025, 2), (60, 148, 2), (60, 149, 2), (136, 6, 2), (22, 4096, 1), (22, 4097, 1), (28, 1793, 1),
+    (65, 3072, 1), (65, 3073, 1), (80, 5, 16), (95, 148, 2), (95, 149, 2), (96, 2368, 1), (96, 2369, 1), (100, 6, 16),
+    (135, 3, 16)])
 def test_matches_the_oracle(ctx, oracle, words, n, rounds):
     rng = random.Random(words * 1000 + n)
     nums = _mix(rng, 32 * words, n)

@@ -229,6 +229,13 @@ def kernel_products_per_test(bits: int, limbs: int) -> int:
     return (bits - 1) * (L * (L + 1) // 2 + L * L + L)
 
 
+def tc_products_per_test(bits: int, limbs: int) -> int:
+    """32x32->64 limb products k_search_tc runs on the integer pipe per test: bits - 1 steps, each the square's
+    L(L+1)/2 cross and diagonal products and 2L for m*w - X*z; the reduction's two products are u8 matrices on
+    the tensor cores."""
+    return (bits - 1) * (limbs * (limbs + 1) // 2 + 2 * limbs)
+
+
 def traffic_per_launch() -> dict | None:
     f = ROOT / "profiles" / "ncu_traffic.json"
     if f.exists():
@@ -456,32 +463,43 @@ def run_ours(args, rank: int, world: int, local_rank: int, dist) -> dict | None:
     bits = (job.K * (m_start + m_inc // 2)).bit_length()
     limbs = job.info["limbs"]
     ppt_formula = products_per_test(bits)
-    ppt = kernel_products_per_test(bits, limbs)
+    one_thread = job.info["tpi"] == 1                  # persistent searches of one thread per number: k_search_tc
+    ppt_mont = kernel_products_per_test(bits, limbs)
+    ppt = tc_products_per_test(bits, limbs) if one_thread else ppt_mont
     kern_s = kern_ms / 1e3
     peak = imad_peak / 2                               # a 32x32->64 product needs a lo and a hi multiply-add
     tr = traffic_per_launch()
+    work = (f"{ppt} limb products on the integer pipe per {bits}-bit test ({bits - 1} steps of {limbs} words: "
+            + ("L(L+1)/2 + 2L each; the reduction is two u8 matrix products on the tensor cores"
+               if one_thread else "L(L+1)/2 + L^2 + L each") + f"), {tests // args.steps} tests per launch; ")
     roof = {"bound": "imad", "achieved": tests * ppt / kern_s / 1e9, "peak": peak / 1e9,
             "unit": "G limb-products/s", "frac": tests * ppt / kern_s / peak,
+            "frac_montgomery": tests * ppt_mont / kern_s / peak,
             "frac_formula": tests * ppt_formula / kern_s / peak,
             "traffic": tr.get("bytes_per_launch") if tr else None,
             "imad_pipe_busy_ncu": tr.get("imad_pipe_busy") if tr else None,
-            "kernel": f"k_search_persistent<{limbs}>",
-            "work": f"{ppt} limb products per {bits}-bit test ({bits - 1} squarings of {limbs} words: "
-                    f"L(L+1)/2 + L^2 + L each), {tests // args.steps} tests per launch; frac_formula uses the "
-                    f"fixed 2*L^2*(B+ceil(B/5)) = {ppt_formula}",
+            "kernel": f"k_search_{'tc' if one_thread else 'persistent_g'}<{limbs}>",
+            "work": work + f"frac_montgomery counts the {ppt_mont} products of Montgomery squarings instead, "
+                    f"frac_formula the fixed 2*L^2*(B+ceil(B/5)) = {ppt_formula}",
             "peak_source": "in-run microbenchmark (pg_measure_imad_peak: 32-bit IMAD/s / 2); "
                            "MEASURED_PEAKS.json has no integer-multiply figure"}
     hbm, hbm_src = hbm_peak()
     esz = 8 if W["max_prime"] >= 2 ** 32 else 4
-    table_b = job.info["num_primes"] * 3 * esz
-    walk_b = job.info["num_primes"] * 8 if W["max_prime"] < 2 ** 32 else 0  # sa, sb of every large prime
+    # primes expecting at most one hit of the window (odd m x (SL + 1) positions) are read with their lattice,
+    # the others with K^-1 and, below 2^32, their walk steps
+    cut = min(W["max_prime"], m_inc // 2 * (W["sl"] + 1))
+    below = (cut / (math.log(cut) - 1)) / (W["max_prime"] / (math.log(W["max_prime"]) - 1))  # share of the primes
+    n_search = round(job.info["num_primes"] * below)
+    n_lat = job.info["num_primes"] - n_search
+    table_b = n_search * 3 * esz + n_lat * 2 * esz
+    walk_b = n_search * 8 + n_lat * 16
     rows_b = m_count * job.info["words_per_m"] * 4
     sieve_b = table_b + walk_b + 2 * rows_b + survivors * 2
     sieve = {"bound": "hbm", "achieved": sieve_b / (sieve_ms / 1e3) / 1e9, "peak": hbm, "unit": "GB/s",
              "frac": sieve_b / (sieve_ms / 1e3) / 1e9 / hbm, "ms_per_window": sieve_ms,
              "bytes_per_window": sieve_b,
-             "work": f"prime table {table_b / 1e9:.3f} GB ({job.info['num_primes']} primes x 3 x {esz} B, read "
-                     f"once) + walk table {walk_b / 1e9:.3f} GB (2 x u32 per prime, read once) + rows "
+             "work": f"prime table {table_b / 1e9:.3f} GB + walk steps and lattices {walk_b / 1e9:.3f} GB (about "
+                     f"{n_search} primes x (3 x {esz} + 8) B, {n_lat} x (2 x {esz} + 16) B, read once) + rows "
                      f"{rows_b / 1e6:.1f} MB written and read once + {survivors} survivors x 2 B; "
                      "time = sieve kernels of a window alone (large-prime search, small-prime tiles and lists)",
              "peak_source": hbm_src}
@@ -497,7 +515,7 @@ def run_ours(args, rank: int, world: int, local_rank: int, dist) -> dict | None:
                    "m_per_gpu_per_step": m_count, "sl": W["sl"], "max_prime": W["max_prime"],
                    "limbs": limbs, "tpi": job.info["tpi"], "small_limit": job.params.small_limit or 65536,
                    "warps_per_sm": args.warps_per_sm, "parallelism": f"weak: {world} disjoint m-windows",
-                   "l2": "inputs larger than L2 (1.18 GB prime tables read every step)"},
+                   "l2": "inputs larger than L2 (2.1 GB of prime tables, walk steps and lattices read every step)"},
         "prp_tests_per_sec": agg["prp_tests_per_sec"],
         "ms_per_step_one_window_alone": max(r["sync_ms"] for r in allr),
         "setup_seconds": setup_s,

@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(128) k_prp_batch(const uint32_t *__restrict__ 
 
 // The bases of one number side by side, 16 lanes a number: for batches so
 // small that the bases in turn would leave the device idle (12 numbers of 22
-// words, 16 bases: 48 ms in turn, the time of one test side by side).
+// words, 16 bases: 48 ms in turn, 2 ms side by side).
 template <int L>
 __global__ void __launch_bounds__(128) k_prp_bases(const uint32_t *__restrict__ cand, uint32_t words, uint32_t n,
                                                    uint32_t rounds, int32_t *__restrict__ out) {

@@ -16,7 +16,7 @@
 //   r   = 2^b * (m*w - X*z)  (mod 2^32L)       2L word products
 // q falls short of T/K by at most 2^-8 + 2^-16 (the cut ends of T and mu, and
 // the columns left out below its guard word), T/K - X*T/(K*n) = m*T/n, and
-// the correction's own rounding is below 2^-5 (tc_usable in pg_dispatch.cu
+// the correction's own rounding is below 2^-5 (pick_tc in pg_dispatch.cu
 // states the sizes), so m*T/n - z lies in [1/32, 1.11) and
 // r / 2^b = m*T - z*n = m*(T - z*K) - z*X in [0, 1.11 n): its low L words hold
 // it, and the next y is below 2.22 n.  r is m*T mod n: with y standing for

@@ -42,16 +42,16 @@ __device__ __forceinline__ int tc_pick_window(const SearchArgs &a, uint32_t kspa
 }
 
 // What bounds it: the integer multiply pipe (L(L+1)/2 + 2L word products a
-// step, 65 % busy at L = 23) together with the register ports that the carry
-// chains and column sums load beside it; the matrix instructions take 16 % of
-// the tensor pipe.  At L = 23 a step takes 2 234 SM-quarter cycles per warp
-// with four CTAs on an SM (1 877 with the matrix round trips left out), at
-// L = 40 5 575 with two; a Montgomery squaring with the reduction on the
-// multiply pipe takes 3 600 and 12 400.  A step alone takes 3 800 cycles (two
-// matrix round trips, the carry chains), so as many CTAs as TMEM and registers
-// hold share an SM.  Searches of P = 257 .. 947 (12 .. 44 words) run 1.2 .. 2.2
-// times as fast as on the one-warp kernel, which keeps the draining launches,
-// the continuations past sl and the sizes pick_tc refuses.
+// step, 65 % busy with four CTAs of L = 23 on an SM, 57 % with two of L = 22)
+// together with the register ports that the carry chains and column sums load
+// beside it; the tensor pipe is 9 % busy and DRAM idle.  At L = 23 a step takes
+// 2 228 SM-quarter cycles per warp with four CTAs on an SM (1 877 with the
+// matrix round trips left out), at L = 40 5 513 with two; a Montgomery squaring
+// with the reduction on the multiply pipe takes 3 600 and 12 400.  A step alone
+// takes 3 800 cycles (two matrix round trips, the carry chains), so as many
+// CTAs as TMEM and registers hold share an SM.  Searches of P = 257 .. 947
+// (12 .. 44 words) run 1.2 .. 2.2 times as fast as on the one-warp kernel,
+// which keeps the draining launches and the sizes pick_tc refuses.
 template <int L>
 __global__ void __launch_bounds__(TC_ROWS, tc_min_blocks(L)) k_search_tc(const __grid_constant__ SearchArgs a) {
     using D = TcDim<L>;

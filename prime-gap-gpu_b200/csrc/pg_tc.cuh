@@ -21,8 +21,8 @@
 // r / 2^b = m*T - z*n = m*(T - z*K) - z*X in [0, 1.11 n): its low L words hold
 // it, and the next y is below 2.22 n.  r is m*T mod n: with y standing for
 // x*m^-1 mod n the step maps x to 2^b * x^2, so a test starts from
-// m^-1 mod n = j*K + (j*X + 1)/m, j = -X^-1 mod m, and compares with +-m^-1 at
-// the end.
+// 2^e * m^-1 mod n = s*K + (s*X + 2^e)/m, s = -2^e * X^-1 mod m, for the leading
+// bits e of the exponent, and compares with +-m^-1 (e = 0) at the end.
 #pragma once
 
 #include "pg_internal.h"
@@ -343,7 +343,49 @@ __device__ __forceinline__ bool tc_inverse(uint32_t m, uint32_t xabs, bool neg, 
     return true;
 }
 
+// y = s*K + (s*X + rho)/m (exact) + q, q in local memory or NULL
+template <int L>
+__device__ __forceinline__ void tc_start(uint32_t (&y)[L], const uint32_t *K, uint32_t s, uint32_t m, int64_t X,
+                                         uint32_t rho, const uint32_t *q) {
+    const int64_t c = ((int64_t)s * X + rho) / (int64_t)m;
+    uint32_t carry = 0;
+#pragma unroll
+    for (int i = 0; i < L; i++) {
+        uint64_t p = (uint64_t)__ldg(K + i) * s + carry;
+        if (q) p += q[i];
+        y[i] = (uint32_t)p;
+        carry = (uint32_t)(p >> 32);
+    }
+    const uint32_t ext = (uint32_t)(c >> 63);
+    y[0] = add_cc(y[0], (uint32_t)c);
+    y[1] = addc_cc(y[1], (uint32_t)((uint64_t)c >> 32));
+#pragma unroll
+    for (int i = 2; i < L; i++) y[i] = i + 1 < L ? addc_cc(y[i], ext) : addc(y[i], ext);
+}
+
 // Helpers on words in local memory, rolled loops: a few calls per test.
+
+// q = floor(2^e / m), e < 32L, m < 2^30; returns 2^e mod m
+template <int L>
+__device__ __noinline__ uint32_t tc_pow2_div(uint32_t *q, uint32_t e, uint32_t m) {
+    const uint64_t inv = ~0ull / m;
+    uint32_t rem = 0;
+    for (int i = L - 1; i >= 0; i--) {
+        uint32_t d = 0;
+        if (i <= (int)(e >> 5)) {
+            const uint64_t v = ((uint64_t)rem << 32) | (i == (int)(e >> 5) ? 1u << (e & 31) : 0u);
+            uint64_t t = __umul64hi(v, inv), r = v - t * m;  // t falls short of v / m by less than 2
+            while (r >= m) {
+                t++;
+                r -= m;
+            }
+            d = (uint32_t)t;
+            rem = (uint32_t)r;
+        }
+        q[i] = d;
+    }
+    return rem;
+}
 
 // x < y
 template <int L>

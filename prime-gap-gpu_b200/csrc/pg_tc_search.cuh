@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(TC_ROWS, tc_min_blocks(L)) k_search_tc(const _
         }
         // the candidates: n = m*K + X, a1 = m^-1 mod n (both in local memory)
         uint32_t n_loc[L], a_loc[L], y[L];
-        uint32_t m = 0, xabs = 0;
+        uint32_t m = 0, xabs = 0, j = 0;
         int B = 0, sbit = 0;
         double ratio = 0;
         const bool prev = s & 1;
@@ -163,22 +163,8 @@ __global__ void __launch_bounds__(TC_ROWS, tc_min_blocks(L)) k_search_tc(const _
                 nd += (double)n_loc[i] * scale;
             }
             ratio = (prev ? (double)xabs : -(double)xabs) / nd;
-            uint32_t j = 0;
             if (tc_inverse(m, xabs, prev, j)) {
-                const int64_t jx = (int64_t)j * xabs;
-                const int64_t c = ((prev ? -jx : jx) + 1) / (int64_t)m;  // exact
-                uint32_t carry = 0;
-#pragma unroll
-                for (int i = 0; i < L; i++) {
-                    const uint64_t p = (uint64_t)__ldg(W.K + i) * j + carry;
-                    y[i] = (uint32_t)p;
-                    carry = (uint32_t)(p >> 32);
-                }
-                const uint32_t ext = (uint32_t)(c >> 63);
-                y[0] = add_cc(y[0], (uint32_t)c);
-                y[1] = addc_cc(y[1], (uint32_t)((uint64_t)c >> 32));
-#pragma unroll
-                for (int i = 2; i < L; i++) y[i] = i + 1 < L ? addc_cc(y[i], ext) : addc(y[i], ext);
+                tc_start<L>(y, W.K, j, m, prev ? -(int64_t)xabs : (int64_t)xabs, 1, nullptr);
 #pragma unroll
                 for (int i = 0; i < L; i++) a_loc[i] = y[i];
             } else {  // gcd(m, X) divides n: composite, as by trial division (past sl, where no sieve row rules it out)
@@ -190,14 +176,34 @@ __global__ void __launch_bounds__(TC_ROWS, tc_min_blocks(L)) k_search_tc(const _
         }
         const long long t_round = clock64();
         const int wb = __reduce_max_sync(FULL, B);
-        if (lane == 0) sh.bmax[tid >> 5] = wb;
+        const bool late = __any_sync(FULL, have && sbit > B - 16);
+        if (lane == 0) sh.bmax[tid >> 5] = wb | (late ? 1 << 16 : 0);
         if (!__syncthreads_or(have)) continue;  // the window's queue ran out under the CTA
         if (tid == 0 && a.settle) atomicAdd(&a.rounds[0], 1u);
-        const int bmax = max(max(sh.bmax[0], sh.bmax[1]), max(sh.bmax[2], sh.bmax[3]));
+        const int b0 = sh.bmax[0], b1m = sh.bmax[1], b2m = sh.bmax[2], b3 = sh.bmax[3];
+        const int bmax = max(max(b0 & 0xffff, b1m & 0xffff), max(b2m & 0xffff, b3 & 0xffff));
+        // The exponent's leading bits cost no step: x = 2^e, e = the bits above
+        // the low bmax - lead ones, is below K (K > 2^(bmax-32), m < 2^30), and
+        // x * m^-1 = s*K + (s*X + 2^e)/m with s = -2^e * X^-1 mod m.  A candidate
+        // whose n - 1 ends above those bits would miss a comparison: then lead = 0.
+        // Seven to nine steps of 461 .. 1 100 saved: P = 337 2.98 -> 2.94 ms, P = 503
+        // 75.9 -> 74.5, P = 811 35.2 -> 34.4; from L = 40 the step itself compiles
+        // to a slower one beside it (P = 907 36.2 -> 36.3), so it is left out there.
+        const bool early = (b0 | b1m | b2m | b3) >> 16;
+        const int lead = L >= 40 || early ? 0 : 31 - __clz(bmax - 32);
+        if (have && lead) {
+            const int sh0 = bmax - lead, wi = sh0 >> 5;
+            const uint32_t lo = n_loc[wi], hi = wi + 1 < L ? n_loc[wi + 1] : 0u;
+            const uint32_t e = wi < L ? __funnelshift_r(lo, hi, sh0 & 31) : 0u;
+            uint32_t q[L];
+            const uint32_t rho = tc_pow2_div<L>(q, e, m);
+            const uint32_t sx = (uint32_t)((uint64_t)j * rho % m);
+            tc_start<L>(y, W.K, sx, m, prev ? -(int64_t)xabs : (int64_t)xabs, rho, q);
+        }
         // y stands for 2^((n-1) >> (b+1)); lanes with fewer bits hold 1 until their top bit
         bool pr = false, done = !have;
-        uint32_t ew = have ? n_loc[(bmax - 1) >> 5] : 0;
-        for (int b = bmax - 1; b >= 0; b--) {
+        uint32_t ew = have ? n_loc[(bmax - 1 - lead) >> 5] : 0;
+        for (int b = bmax - 1 - lead; b >= 0; b--) {
             if (have && (b & 31) == 31) ew = n_loc[b >> 5];
             if (!done && b < sbit) {
                 uint32_t c[L];

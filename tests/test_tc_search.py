@@ -129,3 +129,29 @@ def test_lane_groups_few_sides(pg, m_inc):
         a = job.search(10_000_001, m_inc)
         b = job.wait(job.submit(10_000_001, m_inc, flags=pg.PG_SUBMIT_DRAIN))
     assert np.array_equal(a.prev_gap, b.prev_gap) and np.array_equal(a.next_gap, b.next_gap)
+
+
+@pytest.mark.parametrize("P,d", [(257, 210), (337, 2310), (389, 210), (503, 2190), (811, 210)])
+def test_start_from_the_leading_bits(P, d):
+    """x * m^-1 for x = 2^e, e the exponent's leading bits, in exact arithmetic: the quotient words by the rounded
+    reciprocal, the value and its bound, for candidates shorter than the CTA's longest too."""
+    K, rng = _primorial(P) // d, random.Random(P)
+    for m in [1, 2, 3, (1 << 30) - 1] + [rng.randrange(1, 1 << rng.randrange(2, 31)) for _ in range(60)]:
+        X = 2 * rng.randrange(1, 1 << rng.randrange(1, 23)) * rng.choice([-1, 1])
+        n = m * K + X
+        if n % 2 == 0 or math.gcd(m, abs(X)) > 1:
+            continue
+        bmax = max(n.bit_length(), rng.choice([0, (((1 << 30) - 1) * K).bit_length()]))
+        lead = (bmax - 32).bit_length() - 1
+        e = n >> (bmax - lead)
+        assert e == (n - 1) >> (bmax - lead) and 2 ** e < K
+        inv, rem, q = ((1 << 64) - 1) // m, 0, 0
+        for i in range(e >> 5, -1, -1):
+            v = rem << 32 | ((1 << (e & 31)) if i == e >> 5 else 0)
+            t = v * inv >> 64
+            assert 0 <= v // m - t <= 2 and v // m < 1 << 32
+            q, rem = q << 32 | v // m, v % m
+        s = -pow(X, -1, m) * rem % m if m > 1 else 0
+        assert (s * X + rem) % m == 0
+        y = s * K + (s * X + rem) // m + q
+        assert 0 <= 100 * y < 222 * n and (m * y - (1 << e)) % n == 0

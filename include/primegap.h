@@ -141,6 +141,9 @@ typedef struct {
     uint32_t tpi;             /* threads per number of the PRP kernels */
     uint32_t words_per_m;     /* uint32 words of one sieve row */
     uint32_t side_capacity;   /* longest possible survivor list of one side */
+    uint32_t tc_words;        /* operand words of the search kernel that reduces on the tensor cores;
+                                 0 = the job's sizes are outside its bounds (operands below about 9 or above
+                                 44 words, max_m >= 2^30, tpi > 1): its searches run on the integer pipe */
     uint64_t num_primes;      /* primes in (P, max_prime] */
     uint64_t num_small;       /* of them (plus odd d-primes) sieved per m */
     double k_log;             /* log(K), as _log (gap_common.cpp:44-48) */
@@ -185,7 +188,7 @@ typedef struct {
     uint64_t h2d_bytes;       /* host-to-device bytes copied by the call */
     uint64_t d2h_bytes;       /* device-to-host bytes copied by the call */
     uint32_t graph_launches;  /* CUDA graph launches (the persistent form's window is one graph) */
-    uint32_t pad;
+    uint32_t tc_blocks;       /* thread blocks of the tensor-core search, 0 = another kernel searched */
     uint64_t survivors;       /* candidates the sieve left in [-sl, sl], both sides of every m */
 } pg_search_stats;
 

@@ -88,7 +88,8 @@ class JobInfo(ctypes.Structure):
     _fields_ = [
         ("k_bits", ctypes.c_uint32), ("limbs", ctypes.c_uint32), ("tpi", ctypes.c_uint32),
         ("words_per_m", ctypes.c_uint32),
-        ("side_capacity", ctypes.c_uint32), ("num_primes", ctypes.c_uint64), ("num_small", ctypes.c_uint64),
+        ("side_capacity", ctypes.c_uint32), ("tc_words", ctypes.c_uint32),
+        ("num_primes", ctypes.c_uint64), ("num_small", ctypes.c_uint64),
         ("k_log", ctypes.c_double), ("setup_seconds", ctypes.c_double), ("device_bytes", ctypes.c_uint64),
     ]
 
@@ -100,7 +101,7 @@ class SearchStats(ctypes.Structure):
         ("sieve_ms", ctypes.c_double), ("prp_ms", ctypes.c_double), ("total_ms", ctypes.c_double),
         ("search_kernel_ms", ctypes.c_double), ("kernel_launches", ctypes.c_uint64),
         ("h2d_bytes", ctypes.c_uint64), ("d2h_bytes", ctypes.c_uint64),
-        ("graph_launches", ctypes.c_uint32), ("pad", ctypes.c_uint32), ("survivors", ctypes.c_uint64),
+        ("graph_launches", ctypes.c_uint32), ("tc_blocks", ctypes.c_uint32), ("survivors", ctypes.c_uint64),
     ]
 
     def as_dict(self) -> dict:

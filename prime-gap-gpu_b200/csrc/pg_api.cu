@@ -839,6 +839,7 @@ static int enqueue_windows(Slot &s, int form, uint32_t flags) {
             a.win_next = s.d_wnext;
             a.n_win = (uint32_t)s.parts.size();
             a.failed = &s.d_sc->failed;
+            s.sst.tc_blocks = (uint32_t)s.tc_grid;
             PG_CUDA(cudaMemsetAsync(s.d_wnext, 0, s.parts.size() * 8, s.st));
         }
         s.search = a;
@@ -1316,6 +1317,7 @@ extern "C" int pg_job_get_info(const pg_job *j, pg_job_info *info) {
     info->tpi = j->L >> 16 ? j->L >> 16 : 1;
     info->words_per_m = j->W;
     info->side_capacity = j->cap;
+    info->tc_words = j->tcL;
     info->num_primes = j->T->np;
     info->num_small = j->T->nsmall;
     info->k_log = j->T->k_log;

@@ -306,9 +306,9 @@ int pg_autotune_ex(pg_ctx *ctx, const pg_job_params *base, uint64_t m_start, uin
  * A server takes gap-search requests (any P, d, sl, sieve limit and m range)
  * from any host thread and runs them on one device with continuous batching:
  * a worker thread cuts each request's m range into windows, and packs windows
- * of every admitted request whose operands share a layout into one search
- * launch (one persistent PRP kernel over all their sides), two launches in
- * flight.  Prime tables depend on (P, d, max_prime, small_limit) only and are
+ * of every admitted request whose operands share a layout and a search kernel
+ * (pg_job_info.limbs, .tc_words) into one search launch (one persistent PRP
+ * kernel over all their sides), two launches in flight.  Prime tables depend on (P, d, max_prime, small_limit) only and are
  * shared by every request with that key, whatever its sl or m range.  A
  * request is admitted once its tables are resident; tables that would not fit
  * the device-memory budget wait until idle tables can be evicted (least

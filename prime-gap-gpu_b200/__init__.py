@@ -470,8 +470,8 @@ class Server:
 
     submit() queues a request of any (p, d, sl, max_prime, m range) and
     returns its id at once; a worker thread in the library packs windows of
-    all admitted requests that share an operand layout into common search
-    launches.  wait(id) returns the request's gaps like Job.search."""
+    all admitted requests that share an operand layout and a search kernel into
+    common search launches.  wait(id) returns the request's gaps like Job.search."""
 
     def __init__(self, device: int = 0, hbm_budget: int = 0, batch_m: int = 0, window_m: int = 0,
                  max_windows: int = 0, max_sl: int = 0, small_limit: int = 0, ext_window: int = 0, tpi: int = 0,

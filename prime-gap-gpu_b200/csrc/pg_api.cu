@@ -573,7 +573,7 @@ void pg::slot_reset(Slot &s) {
 
 bool pg::slot_fits(const Slot &s, const pg_job *j, uint64_t nm, uint64_t nodd) {
     if (s.parts.size() >= s.win_cap) return false;
-    if (!s.parts.empty() && (j->L != s.L || j->prm.ext_window != s.ext_window)) return false;
+    if (!s.parts.empty() && (j->L != s.L || j->tcL != s.tcL || j->prm.ext_window != s.ext_window)) return false;
     if (s.nm + nm > s.nm_cap || s.nodd + nodd > s.nodd_cap) return false;
     if (nm * j->W > s.bm_cap) return false;
     const uint64_t stride = std::max(s.stride, j->cap);
@@ -618,7 +618,6 @@ int pg::slot_add(Slot &s, pg_job *j, uint64_t m_start, uint64_t m_inc) {
         s.tcL = j->tcL;
         s.ext_window = p.ext_window;
     }
-    if (s.tcL != j->tcL) s.tcL = 0;
     s.h_win[wid].side0 = 2 * s.nm;
     s.h_win[wid].nsides = 2 * w.nm;
     s.stride = std::max(s.stride, j->cap);

@@ -11,7 +11,7 @@
 //              per-window constants (WinInfo) and two window slots
 //   Slot    -- buffers, stream and in-flight state of one search launch over
 //              one or more windows (of one or several jobs) that share an
-//              operand layout
+//              operand layout and a tensor-core size
 #pragma once
 
 #include <memory>
@@ -118,7 +118,7 @@ struct Slot {
     uint32_t nm = 0;       // m in the slot
     uint64_t nodd = 0;     // odd m in the slot
     uint32_t L = 0;        // operand layout of every window
-    uint32_t tcL = 0;      // operand words of the tensor-core search, 0 = some window cannot use it
+    uint32_t tcL = 0;      // operand words of the tensor-core search of every window, 0 = not used
     bool search_tc = false;  // the search in flight runs on it
     uint32_t stride = 0;   // list stride (largest job capacity)
     uint32_t ext_window = 0;

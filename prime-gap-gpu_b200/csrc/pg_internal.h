@@ -23,7 +23,7 @@ constexpr int PERSIST_THREADS = 32;
 constexpr int TC_MU_WORDS = 48;
 
 // One window of a search launch: the constants of the job it belongs to.  A
-// launch may carry windows of several jobs that share an operand layout; side
+// launch may carry windows of several jobs that share their kernels; side
 // s (m index s >> 1) belongs to window wid[s >> 1], or window 0 when wid is
 // NULL.
 struct WinInfo {

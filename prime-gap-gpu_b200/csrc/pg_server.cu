@@ -10,11 +10,11 @@
 //      built if it fits the budget, after evicting idle sets (no admitted
 //      request uses them) least recently used first; a request whose tables
 //      cannot fit waits, or fails when nothing else holds memory.
-//   2. fill every idle slot with one search launch: the operand layout of
-//      the oldest admitted request with windows left (with preemption: of the
-//      cheapest class with windows left), then windows of every
-//      admitted request of that layout in arrival order until the slot is
-//      full (coprime m, windows, list space).  Windows of different requests
+//   2. fill every idle slot with one search launch: the operand layout and
+//      tensor-core size of the oldest admitted request with windows left (with
+//      preemption: of the cheapest class with windows left), then windows of
+//      every admitted request of that layout and size in arrival order until
+//      the slot is full (coprime m, windows, list space).  Windows of different requests
 //      (different K, sl, rounds) share the launch; the kernels read each
 //      side's constants from its window's WinInfo.
 //   3. finish the oldest launch in flight whose stream is idle: queue its
@@ -318,26 +318,30 @@ struct pg_server {
     // Scheduling class of an operand layout: its words (a test costs ~ words^2 x bits).
     static uint32_t cls(uint32_t layout) { return layout_words(layout); }
 
-    // The layout the next launch packs (0: no windows wait) and the submit
-    // time of its oldest waiting request.  Without preemption: the oldest
-    // waiting request's.  With it: the cheapest class with windows waiting,
-    // so short requests overtake long ones, unless the oldest waiting request
-    // has waited aging_s, which then goes first.
-    uint32_t next_layout(double *since = nullptr) const {
-        uint32_t best = 0;
+    // Windows of both jobs can share a launch (slot_fits): one operand layout
+    // holds several tensor-core sizes, and a launch searches with one of them.
+    static bool same_kernels(const pg_job *a, const pg_job *b) { return a->L == b->L && a->tcL == b->tcL; }
+
+    // The job whose layout and tensor-core size the next launch packs (NULL: no
+    // windows wait) and the submit time of its oldest waiting request.  Without
+    // preemption: the oldest waiting request's.  With it: the cheapest class
+    // with windows waiting, so short requests overtake long ones, unless the
+    // oldest waiting request has waited aging_s, which then goes first.
+    const pg_job *next_job(double *since = nullptr) const {
+        const pg_job *best = nullptr;
         double t_best = -1;
         bool first = true;
         for (uint64_t id : order) {
             const Request &r = reqs.at(id);
             if (r.state != St::ADMITTED || r.next_m >= r.m_end) continue;
             if (first && (!prm.preempt_us || now() - r.t_submit >= aging_s)) {
-                best = r.job->L;
+                best = r.job;
                 t_best = r.t_submit;
                 break;
             }
             first = false;
-            if (!best || cls(r.job->L) < cls(best)) {
-                best = r.job->L;
+            if (!best || cls(r.job->L) < cls(best->L)) {
+                best = r.job;
                 t_best = r.t_submit;
             }
         }
@@ -351,13 +355,13 @@ struct pg_server {
         slot_reset(s);
         ss.placed.clear();
         ss.tabs.clear();
-        const uint32_t layout = next_layout();
-        if (!layout) return false;
+        const pg_job *lead = next_job();
+        if (!lead) return false;
         ss.t_wait = now();
         std::vector<std::pair<uint64_t, std::pair<int, std::string>>> failed;
         for (uint64_t id : order) {
             Request &r = reqs.at(id);
-            if (r.state != St::ADMITTED || r.job->L != layout) continue;
+            if (r.state != St::ADMITTED || !same_kernels(r.job, lead)) continue;
             bool full = false;
             while (r.next_m < r.m_end) {
                 const uint64_t inc = std::min<uint64_t>(r.m_end - r.next_m, prm.window_m);
@@ -390,7 +394,7 @@ struct pg_server {
             // the capacities of create(); fail the request rather than spin
             for (uint64_t id : order) {
                 Request &r = reqs.at(id);
-                if (r.state == St::ADMITTED && r.job->L == layout && r.next_m < r.m_end) {
+                if (r.state == St::ADMITTED && same_kernels(r.job, lead) && r.next_m < r.m_end) {
                     finish(r, PG_ERR_UNSUPPORTED, "window larger than a search launch");
                     break;
                 }
@@ -460,7 +464,7 @@ struct pg_server {
     // With preemption: a persistent launch holds every SM it fits on until its
     // queue drains, so cheaper work would wait behind it.  Once a launch of a
     // cheaper class has been in flight preempt_us, or the next launch's
-    // windows (next_layout) have waited preempt_us with a slot free for them,
+    // windows (next_job) have waited preempt_us with a slot free for them,
     // raise the stop flag of every running launch of a costlier class.
     void maybe_preempt() {
         if (!prm.preempt_us) return;
@@ -472,8 +476,8 @@ struct pg_server {
             if (ss.inflight && !ss.stopping && t - ss.t_wait >= limit) c = std::min(c, cls(ss.s.L));
         }
         double since = -1;
-        const uint32_t L = next_layout(&since);
-        if (L && idle && t - since >= limit) c = std::min(c, cls(L));
+        const pg_job *next = next_job(&since);
+        if (next && idle && t - since >= limit) c = std::min(c, cls(next->L));
         if (c == UINT32_MAX) return;
         for (auto &ss : slot) {
             if (!ss.inflight || ss.stopping || cls(ss.s.L) <= c) continue;
@@ -489,17 +493,17 @@ struct pg_server {
         for (const auto &ss : slot)
             if (ss.inflight && cls(ss.s.L) < cls(x.s.L)) return false;
         if (stop) return true;
-        const uint32_t L = next_layout();
-        return !L || cls(L) >= cls(x.s.L);
+        const pg_job *next = next_job();
+        return !next || cls(next->L) >= cls(x.s.L);
     }
 
     // An idle slot takes new windows unless a stopped launch of the same or a
     // cheaper class waits to resume (it goes first).
     bool may_fill() const {
-        const uint32_t L = next_layout();
-        if (!L) return false;
+        const pg_job *next = next_job();
+        if (!next) return false;
         for (const auto &ss : slot)
-            if (ss.suspended && cls(ss.s.L) <= cls(L)) return false;
+            if (ss.suspended && cls(ss.s.L) <= cls(next->L)) return false;
         return true;
     }
 

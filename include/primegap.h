@@ -132,8 +132,10 @@ typedef struct {
 #define PG_JOB_COMPACT_WALK 0x8u   /* keep the large-prime sieve's walk steps (8 B per prime below
                                       2^32, computed at job creation: 0.8 GB at 2e9) only for the
                                       primes expecting >= 64 hits per window; the others find each
-                                      hit after the first by another modular search.  For short-lived
-                                      jobs (the server sets it for its jobs) */
+                                      hit after the first by another modular search.  Such a job asks
+                                      for no lattices either (16 B per prime, which others keep while
+                                      nothing else needs the memory).  For short-lived jobs (the server
+                                      sets it for its jobs) */
 
 typedef struct {
     uint32_t k_bits;          /* bits of K */

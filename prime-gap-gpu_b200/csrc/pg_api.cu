@@ -19,6 +19,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <shared_mutex>
 #include <string>
 #include <vector>
 
@@ -242,6 +243,66 @@ extern "C" int pg_ctx_destroy(pg_ctx *c) {
     return PG_OK;
 }
 
+// ======================================================== device memory
+
+// The primes' lattices only make the sieve faster, so they give way to every
+// other allocation: device_malloc frees them when memory runs out and tries
+// again, whichever job or context of the process holds them.  A launch that
+// reads them is put on its stream under a LatticeUse, so that freeing them
+// (exclusive, after a device synchronisation) never meets a launch that is
+// still being enqueued; later launches find T.lat NULL and search instead.
+struct LatticeSets {
+    std::shared_mutex mu;
+    std::vector<Tables *> held;
+};
+static LatticeSets &lattice_sets() {
+    static LatticeSets *s = new LatticeSets;  // outlives the last table set
+    return *s;
+}
+struct LatticeUse {
+    std::shared_lock<std::shared_mutex> lock{lattice_sets().mu};
+};
+
+// takes T off the list and frees its lattices (list locked, nothing reads them)
+static uint64_t lattices_drop(Tables *t) {
+    auto &held = lattice_sets().held;
+    held.erase(std::remove(held.begin(), held.end(), t), held.end());
+    cudaFree(t->lat.exchange(nullptr));
+    return t->lat_bytes.exchange(0);
+}
+
+uint64_t pg::lattices_release(const Tables *only) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::unique_lock<std::shared_mutex> lock(lattice_sets().mu);
+    std::vector<Tables *> drop;
+    for (Tables *t : lattice_sets().held)
+        if (only ? t == only : t->device == dev) drop.push_back(t);
+    if (drop.empty() || cudaDeviceSynchronize() != cudaSuccess) return 0;
+    uint64_t bytes = 0;
+    for (Tables *t : drop) bytes += lattices_drop(t);
+    return bytes;
+}
+
+uint64_t pg::lattices_held() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::shared_lock<std::shared_mutex> lock(lattice_sets().mu);
+    uint64_t bytes = 0;
+    for (const Tables *t : lattice_sets().held) bytes += t->device == dev ? t->lat_bytes.load() : 0;
+    return bytes;
+}
+
+static cudaError_t device_malloc(void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();  // must not surface in a later call
+    if (e == cudaErrorMemoryAllocation && lattices_release(nullptr)) {
+        e = cudaMalloc(p, bytes);
+        if (e != cudaSuccess) cudaGetLastError();
+    }
+    return e;
+}
+
 // ================================================================== PRP
 
 extern "C" int pg_prp_batch_device(pg_ctx *c, const uint32_t *d_limbs, uint32_t n, uint32_t words, uint32_t rounds,
@@ -272,14 +333,14 @@ extern "C" int pg_prp_batch(pg_ctx *c, const uint32_t *limbs, uint32_t n, uint32
         cudaFree(c->d_cand);
         c->d_cand = nullptr;
         c->cand_cap = 0;
-        PG_CUDA(cudaMalloc((void **)&c->d_cand, cb));
+        PG_CUDA(device_malloc((void **)&c->d_cand, cb));
         c->cand_cap = cb;
     }
     if (rb > c->res_cap) {
         cudaFree(c->d_res);
         c->d_res = nullptr;
         c->res_cap = 0;
-        PG_CUDA(cudaMalloc((void **)&c->d_res, rb));
+        PG_CUDA(device_malloc((void **)&c->d_res, rb));
         c->res_cap = rb;
     }
     PG_CUDA(cudaMemcpyAsync(c->d_cand, limbs, cb, cudaMemcpyHostToDevice, c->stream));
@@ -295,10 +356,9 @@ extern "C" int pg_prp_batch(pg_ctx *c, const uint32_t *limbs, uint32_t n, uint32
 template <typename T>
 static int dalloc(uint64_t &acct, T **p, size_t count) {
     const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-    cudaError_t e = cudaMalloc((void **)p, bytes);
+    cudaError_t e = device_malloc((void **)p, bytes);
     if (e != cudaSuccess) {
         *p = nullptr;
-        cudaGetLastError();
         return fail(e == cudaErrorMemoryAllocation ? PG_ERR_NOMEM : PG_ERR_CUDA, "cudaMalloc(%zu): %s", bytes,
                     cudaGetErrorString(e));
     }
@@ -308,7 +368,11 @@ static int dalloc(uint64_t &acct, T **p, size_t count) {
 
 pg::Tables::~Tables() {
     cudaSetDevice(device);
-    void *ptrs[] = {d_sq, d_sr, d_sbar, d_tq, d_lp, d_lc, d_lcinv, d_lat};
+    if (lat) {
+        std::unique_lock<std::shared_mutex> lock(lattice_sets().mu);
+        lattices_drop(this);
+    }
+    void *ptrs[] = {d_sq, d_sr, d_sbar, d_tq, d_lp, d_lc, d_lcinv};
     for (void *p : ptrs) cudaFree(p);
 }
 
@@ -329,7 +393,7 @@ uint64_t pg::tables_bytes_estimate(const pg_job_params &p) {
     return (uint64_t)(3.0 * esz * pi_hi + 16.0 * q1 + (1u << 20));
 }
 
-static int tables_build(pg::Tables &T, const pg_job_params &p, uint64_t lat_bytes, cudaStream_t st) {
+static int tables_build(pg::Tables &T, const pg_job_params &p, cudaStream_t st) {
     // ---- K = P#/d
     std::vector<uint32_t> upto_p = host_primes(p.p);
     T.K.assign(1, 1);
@@ -471,21 +535,38 @@ static int tables_build(pg::Tables &T, const pg_job_params &p, uint64_t lat_byte
             cudaFree(oci);
             cudaFree(dep);
         }
-        if (e == cudaSuccess && acc && acc <= lat_bytes / sizeof(LatC)) {
-            uint64_t extra = 0;
-            if (!dalloc(extra, &T.d_lat, acc)) {
-                e = launch_lattices(T.d_lp, T.d_lc, T.d_lcinv, T.wide, acc, T.d_lat, st);
-                T.bytes += extra;
-            }
-            g_last_error.clear();
-        }
         free_scratch();
         if (e != cudaSuccess) return fail(PG_ERR_CUDA, "prime tables: %s", cudaGetErrorString(e));
     }
     return PG_OK;
 }
 
-int pg::tables_get(pg_ctx *c, const pg_job_params &p, std::shared_ptr<Tables> &out, uint64_t lat_bytes) {
+// The lattices of T's primes, where they fit in `room` bytes and in half of the
+// free device memory (the rest of the process allocates beside them).
+static int lattices_add(pg::Tables &T, uint64_t room, cudaStream_t st) {
+    const uint64_t bytes = T.np * sizeof(LatC);
+    size_t free_b = 0, total_b = 0;
+    if (!bytes || T.lat || bytes > room || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b / 2)
+        return PG_OK;
+    LatC *lat = nullptr;
+    if (cudaMalloc((void **)&lat, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return PG_OK;
+    }
+    cudaError_t e = launch_lattices(T.d_lp, T.d_lc, T.d_lcinv, T.wide, T.np, lat, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+        cudaFree(lat);
+        return fail(PG_ERR_CUDA, "lattices: %s", cudaGetErrorString(e));
+    }
+    std::unique_lock<std::shared_mutex> lock(lattice_sets().mu);
+    T.lat = lat;
+    T.lat_bytes = bytes;
+    lattice_sets().held.push_back(&T);
+    return PG_OK;
+}
+
+int pg::tables_get(pg_ctx *c, const pg_job_params &p, std::shared_ptr<Tables> &out, uint64_t lat_room) {
     const uint32_t q1 = small_bound(p);
     std::lock_guard<std::mutex> lock(c->tables_mu);
     auto &v = c->tables;
@@ -494,7 +575,7 @@ int pg::tables_get(pg_ctx *c, const pg_job_params &p, std::shared_ptr<Tables> &o
         std::shared_ptr<Tables> t = w.lock();
         if (t && t->p == p.p && t->d == p.d && t->max_prime == p.max_prime && t->q1 == q1) {
             out = t;
-            return PG_OK;
+            return lattices_add(*t, lat_room, c->stream);
         }
     }
     const auto t0 = std::chrono::steady_clock::now();
@@ -504,7 +585,8 @@ int pg::tables_get(pg_ctx *c, const pg_job_params &p, std::shared_ptr<Tables> &o
     t->d = p.d;
     t->max_prime = p.max_prime;
     t->q1 = q1;
-    int rc = tables_build(*t, p, lat_bytes, c->stream);
+    int rc = tables_build(*t, p, c->stream);
+    if (!rc) rc = lattices_add(*t, lat_room, c->stream);
     if (rc) return rc;  // t frees what it holds
     t->setup_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     v.push_back(t);
@@ -690,12 +772,12 @@ static uint64_t seg_bands(const pg_job *j, uint64_t split, uint64_t nodd, SegBan
 // most LAT_HITS hits in the window.
 static uint64_t lattice_first(const pg_job *j, uint64_t m0, uint64_t nodd) {
     const pg::Tables &T = *j->T;
-    if (!T.d_lat || m0 >= (1ull << 30) || nodd >= (1ull << 30)) return T.np;
+    if (!T.lat || m0 >= (1ull << 30) || nodd >= (1ull << 30)) return T.np;
     return table_index_at(T, (double)nodd * (2.0 * j->sly + 1) / LAT_HITS);
 }
 
 // sieve of one window of the slot into its rows of lists (compact) or into
-// the bitmap rows (the slot's first window only)
+// the bitmap rows (the slot's first window only); called under a LatticeUse
 static int run_sieve(Slot &s, const WinPart &w, bool compact) {
     const pg_job *j = w.job;
     const pg::Tables &T = *j->T;
@@ -721,7 +803,7 @@ static int run_sieve(Slot &s, const WinPart &w, bool compact) {
     int nb = 0;
     const uint64_t search_first = seg_bands(j, split, w.nodd, bands, &nb);
     const uint64_t lat_first = std::max(search_first, lattice_first(j, w.m0, w.nodd));
-    la.lat = lat_first < T.np ? T.d_lat : nullptr;
+    la.lat = lat_first < T.np ? T.lat.load() : nullptr;
     PG_CUDA(launch_sieve_large(la, T.wide, split, bands, nb, search_first, lat_first, s.st));
     s.sst.kernel_launches += (split > 0) + (nb > 0) + (search_first < lat_first) + (lat_first < T.np);
     SieveArgs sa{};
@@ -963,6 +1045,7 @@ static int round_blocks(Slot &s, int most, int step, double slope, double per) {
 }
 
 int pg::slot_enqueue(Slot &s, int form, uint32_t flags, bool graph) {
+    const LatticeUse use;
     s.fin_active = false;
     s.sst.m_count = s.nm;
     s.sst.h2d_bytes = (uint64_t)s.nm * 8 + (uint64_t)s.nodd * 4 + s.parts.size() * sizeof(WinInfo) +
@@ -1153,7 +1236,7 @@ extern "C" int pg_job_destroy(pg_job *j) {
 
 static int job_build(pg_job *j) {
     const pg_job_params &p = j->prm;
-    int rc = tables_get(j->ctx, p, j->T);
+    int rc = tables_get(j->ctx, p, j->T, p.flags & PG_JOB_COMPACT_WALK ? 0 : ~0ull);
     if (rc) return rc;
     const pg::Tables &T = *j->T;
     // every candidate must exceed max_prime (divisible then means composite)
@@ -1233,7 +1316,7 @@ static int job_build(pg_job *j) {
         double pmax = 4294967296.0;
         if (p.flags & PG_JOB_COMPACT_WALK)
             pmax = (double)j->nodd_cap * (2.0 * j->sly + 1) / SEG_HITS;
-        else if (T.d_lat && p.max_m < (1ull << 30))
+        else if (T.lat && p.max_m < (1ull << 30))
             pmax = (double)j->nodd_cap * (2.0 * j->sly + 1) / LAT_HITS;
         // table_index_at keeps the whole segment holding pmax: with primes above
         // 2^32 in the table, stop a segment early so every kept prime is below 2^32
@@ -1321,7 +1404,7 @@ extern "C" int pg_job_get_info(const pg_job *j, pg_job_info *info) {
     info->num_small = j->T->nsmall;
     info->k_log = j->T->k_log;
     info->setup_seconds = j->setup_s;
-    uint64_t b = j->own_bytes + j->T->bytes;
+    uint64_t b = j->own_bytes + j->T->bytes + j->T->lat_bytes;
     for (const auto &s : j->slot) b += s.bytes;
     info->device_bytes = b;
     return PG_OK;
@@ -1371,7 +1454,10 @@ extern "C" int pg_sieve_interval(pg_job *j, uint64_t m_start, uint64_t m_inc, ui
     if ((rc = job_window(j, s, m_start, m_inc))) return rc;
     if (s.nm == 0) return PG_OK;
     if ((rc = slot_upload(s))) return rc;
-    if ((rc = run_sieve(s, s.parts[0], false))) return rc;
+    {
+        const LatticeUse use;
+        if ((rc = run_sieve(s, s.parts[0], false))) return rc;
+    }
     if (bitmaps) PG_CUDA(cudaMemcpyAsync(bitmaps, s.d_bitmaps, (size_t)s.nm * j->W * 4, cudaMemcpyDeviceToHost, s.st));
     PG_CUDA(cudaStreamSynchronize(s.st));
     if (ms) std::memcpy(ms, s.h_ms, (size_t)s.nm * 8);

@@ -14,6 +14,7 @@
 //              operand layout and a tensor-core size
 #pragma once
 
+#include <atomic>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -58,7 +59,9 @@ struct Tables {
     uint32_t *d_tq = nullptr;   // trial primes 3, 5, 7, ...
     std::vector<uint32_t> tr;   // their residues (-(K mod q)/2) mod q
     void *d_lp = nullptr, *d_lc = nullptr, *d_lcinv = nullptr;
-    LatC *d_lat = nullptr;  // reduced lattices of the primes; NULL = not kept (memory)
+    // reduced lattices of the primes, NULL = not kept; read under a LatticeUse
+    std::atomic<LatC *> lat{nullptr};
+    std::atomic<uint64_t> lat_bytes{0};  // not in bytes
     uint64_t np = 0;
     bool wide = false;
     // prime-table index of each sieve segment (segment s starts at value seg_v0 + s * seg_span)
@@ -70,12 +73,17 @@ struct Tables {
 };
 
 // The tables of (p, d, max_prime, small_limit) on ctx: a live copy shared with
-// other jobs, else a new build.  The lattices (16 B a prime) are kept where
-// they take no more than lat_bytes and the device has room.
-int tables_get(pg_ctx *c, const pg_job_params &p, std::shared_ptr<Tables> &out, uint64_t lat_bytes = ~0ull);
+// other jobs, else a new build.  The lattices (16 B a prime) are added where
+// they take no more than lat_room bytes and half of the free device memory.
+int tables_get(pg_ctx *c, const pg_job_params &p, std::shared_ptr<Tables> &out, uint64_t lat_room);
 // Device bytes a build of those tables would take without the lattices (an
 // upper estimate).
 uint64_t tables_bytes_estimate(const pg_job_params &p);
+// Frees the lattices of one table set, or of every set on the current device
+// (NULL), once the device has finished what was enqueued; the bytes freed.
+uint64_t lattices_release(const Tables *only);
+// Bytes that lattices_release(NULL) would free.
+uint64_t lattices_held();
 
 // One window of a slot.
 struct WinPart {

@@ -161,8 +161,15 @@ struct pg_server {
         return b;
     }
 
+    // lattices held beside resident(): they give way to tables (admit)
+    uint64_t lattices() const {
+        uint64_t b = 0;
+        for (const auto &kv : tables) b += kv.second.T->lat_bytes;
+        return b;
+    }
+
     void note_bytes() {
-        st.resident_bytes = resident();
+        st.resident_bytes = resident() + lattices();
         st.peak_bytes = std::max(st.peak_bytes, st.resident_bytes);
     }
 
@@ -268,10 +275,14 @@ struct pg_server {
                     continue;  // wait for memory
                 }
                 std::shared_ptr<Tables> T;
-                // the lattices may take a quarter of what the budget leaves, so
-                // they never keep another table set out for long
-                const uint64_t spare = (prm.hbm_budget - resident() - need) / 4;
+                // the lattices may take a quarter of what the budget leaves, and
+                // those of the sets in place go first where it would not hold both
+                // (this thread alone changes the table sets)
                 lk.unlock();
+                for (auto t = tables.begin(); t != tables.end() && resident() + lattices() + need > prm.hbm_budget; ++t)
+                    lattices_release(t->second.T.get());
+                const uint64_t want = resident() + lattices() + need;
+                const uint64_t spare = want < prm.hbm_budget ? (prm.hbm_budget - want) / 4 : 0;
                 int rc = tables_get(ctx, tp, T, spare);
                 std::string err = rc ? pg_last_error() : "";
                 lk.lock();
@@ -641,7 +652,7 @@ extern "C" int pg_server_create(int device, const pg_server_params *params, pg_s
             pg_ctx_destroy(c);
             return fail(PG_ERR_CUDA, "pg_server_create: cudaMemGetInfo: %s", cudaGetErrorString(e));
         }
-        p.hbm_budget = free_b / 4 * 3;
+        p.hbm_budget = (free_b + lattices_held()) / 4 * 3;
     }
     pg_server *srv = new pg_server();
     srv->ctx = c;

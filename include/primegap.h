@@ -107,9 +107,10 @@ typedef struct {
                               0 = default (65536) */
     uint32_t ext_window;   /* extension positions past sl tried in the first pass; 0 = 64 */
     uint32_t flags;        /* PG_JOB_* */
-    uint32_t search_hits;  /* 0 = every large prime above 2*sl+1 is sieved by modular search
-                              (default); n > 0 keeps primes expecting >= n hits per window on
-                              the kernel that steps every X */
+    uint32_t search_hits;  /* 0 = every large prime above 2*sl+1 is sieved by modular search or,
+                              expecting at most one hit per window, by its lattice (default);
+                              n > 0 keeps primes expecting >= n hits per window on the kernel
+                              that steps every X */
     uint32_t tpi;          /* threads per number of the PRP kernels: 0 = automatic (one
                               thread up to 48 words, then groups), 1, or a group size 4 / 8 / 16 */
     double confirm_merit;  /* record confirmation (the double-check of overflow.cpp:164-177):
@@ -124,7 +125,7 @@ typedef struct {
 
 /* large-prime sieve: 0 = automatic, else force one method */
 #define PG_JOB_LARGE_STEP   0x1u   /* step every X for every prime */
-#define PG_JOB_LARGE_SEARCH 0x2u   /* modular search for the next hit */
+#define PG_JOB_LARGE_SEARCH 0x2u   /* modular search for the next hit (no lattices) */
 #define PG_JOB_NO_GRAPH     0x4u   /* launch the persistent form's kernels one by one
                                       instead of as one CUDA graph per window; pg_job_create
                                       then returns without waiting for the device (the job's

@@ -718,9 +718,9 @@ static uint64_t table_index_at(const pg::Tables &T, double v) {
     return T.seg_off[(size_t)s];
 }
 
-// First prime-table index sieved by modular search rather than by stepping
-// every Y.  The search needs p > 2 sly + 1 (one hit per m); by default every
-// such prime is searched (with the hit walk, stepping is slower at any split
+// First prime-table index sieved by modular search (or lattices) rather than by
+// stepping every Y.  The search needs p > 2 sly + 1 (one hit per m); by default
+// every such prime is searched (with the hit walk, stepping is slower at any split
 // on the P=503 window); search_hits > 0 keeps primes expecting at least that
 // many hits, nodd * (2 sly + 1) / p, on the stepping kernel.
 static uint64_t large_split(const pg_job *j, uint64_t nodd) {
@@ -769,10 +769,10 @@ static uint64_t seg_bands(const pg_job *j, uint64_t split, uint64_t nodd, SegBan
 }
 
 // First prime-table index sieved by the primes' lattices: those expecting at
-// most LAT_HITS hits in the window.
+// most LAT_HITS hits in the window; none for a job that forces the search.
 static uint64_t lattice_first(const pg_job *j, uint64_t m0, uint64_t nodd) {
     const pg::Tables &T = *j->T;
-    if (!T.lat || m0 >= (1ull << 30) || nodd >= (1ull << 30)) return T.np;
+    if (!T.lat || (j->prm.flags & PG_JOB_LARGE_SEARCH) || m0 >= (1ull << 30) || nodd >= (1ull << 30)) return T.np;
     return table_index_at(T, (double)nodd * (2.0 * j->sly + 1) / LAT_HITS);
 }
 
@@ -1236,7 +1236,8 @@ extern "C" int pg_job_destroy(pg_job *j) {
 
 static int job_build(pg_job *j) {
     const pg_job_params &p = j->prm;
-    int rc = tables_get(j->ctx, p, j->T, p.flags & PG_JOB_COMPACT_WALK ? 0 : ~0ull);
+    const uint32_t no_lattices = PG_JOB_COMPACT_WALK | PG_JOB_LARGE_STEP | PG_JOB_LARGE_SEARCH;
+    int rc = tables_get(j->ctx, p, j->T, p.flags & no_lattices ? 0 : ~0ull);
     if (rc) return rc;
     const pg::Tables &T = *j->T;
     // every candidate must exceed max_prime (divisible then means composite)
@@ -1316,7 +1317,7 @@ static int job_build(pg_job *j) {
         double pmax = 4294967296.0;
         if (p.flags & PG_JOB_COMPACT_WALK)
             pmax = (double)j->nodd_cap * (2.0 * j->sly + 1) / SEG_HITS;
-        else if (T.lat && p.max_m < (1ull << 30))
+        else if (T.lat && !(p.flags & PG_JOB_LARGE_SEARCH) && p.max_m < (1ull << 30))
             pmax = (double)j->nodd_cap * (2.0 * j->sly + 1) / LAT_HITS;
         // table_index_at keeps the whole segment holding pmax: with primes above
         // 2^32 in the table, stop a segment early so every kept prime is below 2^32

@@ -250,9 +250,11 @@ int pg_next_prime_noalloc(const uint32_t *d_numbers, uint32_t n, uint32_t words,
  * would remain busy, handing their SMs to the next window (for callers that
  * keep another window submitted; a lone window finishes later with it);
  * D = (flags >> 8) & 0xff, 0 = 4.  PG_SUBMIT_WARPS_PER_SM(w) caps the PRP
- * kernel at w resident warps per SM (0 = as many as fit; rounded up to whole
- * thread blocks of 4 warps where the search runs on the tensor cores), leaving
- * room for the next window's kernels to run beside it.  pg_search() is submit + wait. */
+ * kernel at w resident warps per SM (0 = as many as fit), leaving room for the
+ * next window's kernels to run beside it; where the search runs on the tensor
+ * cores (pg_job_info.tc_words), w is rounded up to whole thread blocks of 4
+ * warps, but a cap below what fits leaves room for at least one more block if
+ * two fit.  pg_search() is submit + wait. */
 #define PG_SEARCH_SLOTS 2
 #define PG_SUBMIT_DRAIN 0x1u
 #define PG_SUBMIT_DRAIN_LANES(d) (((uint32_t)(d) & 0xffu) << 8)
@@ -284,8 +286,9 @@ int pg_autotune(pg_ctx *ctx, const pg_job_params *base, uint64_t m_start, uint64
  *      262144;
  *   3. the PRP kernel's warps per SM (PG_SUBMIT_WARPS_PER_SM): 0 (all that
  *      fit), 4, 6, 8, 10, 12, each over max(2 x reps, 8) passes (a short
- *      sample favours full occupancy), then the two fastest once more, and
- *      the mean of their two timings decides;
+ *      sample favours full occupancy; caps that give the same launch count as
+ *      one, the lowest), then the two fastest once more, and the mean of their
+ *      two timings decides;
  *   4. with PG_TUNE_WINDOW, the m per window: m_inc, m_inc / 2, m_inc / 4.
  * The exponentiation window has no knob: the base-2 test multiplies by
  * doublings, never by a table entry.  Each setting runs one warm-up pass and

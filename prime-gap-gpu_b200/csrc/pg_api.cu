@@ -1044,6 +1044,18 @@ static int round_blocks(Slot &s, int most, int step, double slope, double per) {
     return best;
 }
 
+// CTAs per SM of a tensor-core search capped at w warps per SM, where `most`
+// fit.  The cap means that another launch runs beside this one, so it is
+// rounded up to whole CTAs of 4 warps (P = 503, two windows of 200 000 m in
+// flight at a cap of 6: 77.4 ms a window at 1.5 CTAs per SM, 71.0 at 2), except
+// that a cap below what fits leaves room for a CTA (P = 907, where two fit:
+// 42.4 ms at 1, 47.0 at 2).
+static int tc_cap_blocks(int most, uint32_t w) {
+    const int up = ((int)w + 3) / 4;
+    if (up < most) return up;
+    return (int)w < 4 * most ? std::max(most - 1, 1) : most;
+}
+
 int pg::slot_enqueue(Slot &s, int form, uint32_t flags, bool graph) {
     const LatticeUse use;
     s.fin_active = false;
@@ -1059,12 +1071,7 @@ int pg::slot_enqueue(Slot &s, int form, uint32_t flags, bool graph) {
     if (s.tcL) {
         const int most = tc_blocks_per_sm(s.tcL);
         if (wps)
-            // another launch runs beside this one: the cap in whole CTAs of 4
-            // warps, and at most half of those that fit, so both find room
-            // (P = 503, two windows of 200 000 m in flight at a cap of 6: 77.4 ms
-            // a window at 1.5 CTAs per SM, 71.0 at 2; P = 907, where two fit:
-            // 42.4 ms at 1, 47.0 at 2)
-            s.tc_grid = sms * std::min(((int)wps + 3) / 4, (most + 1) / 2);
+            s.tc_grid = sms * tc_cap_blocks(most, wps);
         else
             s.tc_grid = sms * (s.shared ? most : round_blocks(s, most, 1, s.tcL < 20 ? 0.33 : s.tcL < 30 ? 0.43 : 0.37, 128));
     } else if ((s.L >> 16) && !wps && !s.shared && form == PG_SEARCH_PERSISTENT && !(flags & PG_SUBMIT_DRAIN)) {
@@ -1675,7 +1682,9 @@ extern "C" int pg_autotune_ex(pg_ctx *c, const pg_job_params *base, uint64_t m_s
     // per cent, and a sample of one or two windows favours full occupancy
     // (its windows start side by side and end alone), so every cap is timed
     // over at least 8 windows on one job, then the two best once more, and
-    // the mean of their two timings decides.
+    // the mean of their two timings decides.  Caps that the job's kernel turns
+    // into the same launch are one candidate, the lowest of them, with the mean
+    // of their timings: which of them came out ahead would be noise.
     const uint32_t caps[] = {0, 4, 6, 8, 10, 12};
     const pg_job_params tuned = best.params;
     {
@@ -1683,13 +1692,25 @@ extern "C" int pg_autotune_ex(pg_ctx *c, const pg_job_params *base, uint64_t m_s
         int rc = pg_job_create(c, &tuned, &j);
         if (rc) return rc;
         const uint32_t passes = std::max(2 * reps, 8u);
-        std::vector<std::pair<double, uint32_t>> by_cap;
+        struct Launch {
+            int blocks;  // per SM, -1 = no cap
+            uint32_t cap, n;
+            double sum;
+        };
+        std::vector<Launch> launches;
+        const int fit = j->tcL ? tc_blocks_per_sm(j->tcL) : search_grid(j->L, c->device) / c->sms;
         for (uint32_t w : caps) {
             double v = 0;
             if ((rc = time_pipelined(j, m_start, m_inc, m_inc, PG_SUBMIT_WARPS_PER_SM(w), passes, &v))) break;
-            by_cap.push_back({v, w});
+            const int blocks = !w ? -1 : j->tcL ? tc_cap_blocks(fit, w) : std::min((int)w, fit);
+            auto same = std::find_if(launches.begin(), launches.end(), [&](const Launch &l) { return l.blocks == blocks; });
+            if (same == launches.end()) same = launches.insert(launches.end(), Launch{blocks, w, 0, 0.0});
+            same->n++;
+            same->sum += v;
             settings++;
         }
+        std::vector<std::pair<double, uint32_t>> by_cap;
+        for (const Launch &l : launches) by_cap.push_back({l.sum / l.n, l.cap});
         std::sort(by_cap.rbegin(), by_cap.rend());
         for (size_t k = 0; k < 2 && !rc; k++) {
             double v = 0;

@@ -173,6 +173,12 @@ struct LatC {
     int32_t w;
 };
 constexpr uint32_t LAT_W = 1u << 13;
+// A window's range of t is computed from reciprocals good to 2^-38 and widened
+// by LAT_EDGE, which covers their error while M < LAT_MAX_M: |t| stays near M,
+// so it is off by at most M * 2^-38 + 2^-26 (lattice_hits).  M <= 2p / LAT_W,
+// so every prime below 2^36 qualifies; the others' are kept out.
+constexpr uint32_t LAT_MAX_M = 1u << 24;
+constexpr double LAT_EDGE = 1e-4;
 constexpr double LAT_HITS = 1.0;
 
 // Primes of the large-prime table processed by the segmented kernel in one

@@ -676,7 +676,8 @@ __device__ __forceinline__ void sieve_prime(const LargeArgs &a, const uint32_t *
     }
 }
 
-// 1/x to about 2^-40 (x from 1 to 2^40)
+// 1/x to 2^-38 (x from 1 to 2^40): the approximation reads and returns the top
+// 32 bits, each cut 2^-20, and one Newton step squares its error
 __device__ __forceinline__ double fast_rcp(double x) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
@@ -688,8 +689,10 @@ __device__ __forceinline__ double fast_rcp(double x) {
 // [b - W, b].  t = (M*S - max(w, 0)*x) / p (w > 0) or (M*S + |w|*x) / p, so t
 // runs over an interval about (W + |w| J / M) M / p wide (a point or two where
 // hits are few), and for each t the points are M apart in x.  The
-// interval's ends and Q come from doubles with room for their rounding;
-// x and S are exact integers, checked.
+// interval's ends and Q come from doubles with room for their rounding: the
+// ends are at most M + |w| J / p, J / p below 1 / W, so with reciprocals good to
+// 2^-38 and M < LAT_MAX_M they are off by less than LAT_EDGE.  x and S are exact
+// integers, checked.
 //
 // m0 < 2^30 here, so m0 * (K/2) / p < 2^30 and its quotient from the fast
 // reciprocal is within one.
@@ -706,8 +709,8 @@ __device__ __forceinline__ void lattice_hits(const LargeArgs &a, const uint32_t 
     const double rM = (double)M * inv, edge = (double)l.w * (double)J * inv;
     const double hi = rM * (double)b + (edge < 0 ? -edge : 0.0);
     const double lo = rM * ((double)b - (double)W) - (edge > 0 ? edge : 0.0);
-    int32_t t = __double2int_rd(hi + 1e-4);
-    const int32_t t0 = __double2int_ru(lo - 1e-4);
+    int32_t t = __double2int_rd(hi + LAT_EDGE);
+    const int32_t t0 = __double2int_ru(lo - LAT_EDGE);
     if (t < t0) return;
     int32_t Q = __double2int_ru((double)t * (double)l.inc * fast_rcp((double)M));
     int32_t x = (int32_t)((uint32_t)Q * l.M - (uint32_t)t * l.inc);  // within one of its Q: |x| < 2^31
@@ -844,7 +847,7 @@ __global__ void __launch_bounds__(256) k_lattices(const T *pt, const T *ct, cons
                 dec = beta + d * alpha;
                 w = -(int32_t)alpha;
             }
-            if (M < (1u << 30) && dec < (1ull << 32)) l = LatC{(uint32_t)M, (uint32_t)inc, (uint32_t)dec, w};
+            if (M < LAT_MAX_M && dec < (1ull << 32)) l = LatC{(uint32_t)M, (uint32_t)inc, (uint32_t)dec, w};
         }
     }
     out[i] = l;

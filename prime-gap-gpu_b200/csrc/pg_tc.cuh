@@ -45,6 +45,10 @@ struct TcDim {
     static constexpr int N2 = (4 * L + 15) / 16 * 16;
     static constexpr int NMAX = N1 > N2 ? N1 : N2;
     static constexpr int COLS = NMAX <= 32 ? 32 : NMAX <= 64 ? 64 : NMAX <= 128 ? 128 : 256;  // TMEM columns
+    // a column of D sums at most 4 NT products of two bytes; tc_words needs a
+    // pair of columns with what moved up from the pair below in 32 bits (so up
+    // to 256 bytes, L = 60; 192 at L = 44)
+    static_assert(257ull * (4 * NT) * 255 * 255 + 65535 <= 0xffffffffull, "columns too large for tc_words");
     static constexpr int A_BYTES = TC_ROWS * (K1 > K2 ? K1 : K2);
     static constexpr int SMEM = A_BYTES + N1 * K1 + N2 * K2;
 };
@@ -168,9 +172,9 @@ __device__ __forceinline__ void tc_square(const uint32_t (&x)[L], uint32_t (&T)[
 }
 
 // NW words from the byte columns of the D matrix from column 0 on: four
-// columns (each below 2^23) make a word.  With p0 = c0 + c1*2^8 and
-// p1 = c2 + c3*2^8 (both below 2^31) the value is the sum of two word strings,
-// p0 plus the high half of the p1 below it, and p1's low half moved up: one
+// columns (each below 2^24, TcDim) make a word.  With p0 = c0 + c1*2^8 and
+// p1 = c2 + c3*2^8 the value is the sum of two word strings, p0 plus the high
+// half of the p1 below it (below 2^32, TcDim), and p1's low half moved up: one
 // carry chain, so no 64-bit multiply (p1 * 2^16 + p0) adds to the multiply
 // pipe's load: 2507 -> 2234 cycles a step at L = 23.  Columns are read 16 at a
 // time, three reads in flight.

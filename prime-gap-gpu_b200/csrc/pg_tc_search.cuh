@@ -219,7 +219,12 @@ __global__ void __launch_bounds__(TC_ROWS, tc_min_blocks(L)) k_search_tc(const _
             if (!tc_step<L>(S, y, m, xabs, prev ? 0xffffffffu : 0u, ratio, (ew >> (b & 31)) & 1u)) break;
         }
         if (!__syncthreads_and(S.ok)) {
-            if (tid == 0) atomicExch(a.failed, 1u);
+            if (tid == 0) {
+                atomicExch(a.failed, 1u);
+                // the matrix instruction that was given up on may still read shared
+                // memory and write TMEM: once more the limit before both are freed
+                tc_wait(S.mbar, S.phase ^ 1u);
+            }
             break;
         }
         if (have) {

@@ -61,8 +61,9 @@ uint32_t pick_limbs(uint32_t words) { return pick_layout(32 * words, 0); }
 // Bases run side by side while 16 lanes (or groups) per number still finish in
 // the time of one test: up to 16 384 tests of one thread each (22 words:
 // 2.05 ms for 16 and for 16 384 tests), or 18 944 lanes in groups (one warp per
-// SM quarter).  Few tests of more than 16 words take a group of lanes per
+// SM quarter).  Few tests of more than 20 words take a group of lanes per
 // number; the layouts were timed against one thread per number:
+//   21 words 8 x 3: 1.58, 1.60, 1.79 ms at 64, 2 048, 4 096 tests (1.85 to 1.95)
 //   22 words 8 x 3: 1.66, 1.87, 2.53 ms at 2 048, 4 096, 8 192 tests (2.05 at each)
 //   32 words 16 x 3: 3.58, 4.19, 6.27 ms at 512, 2 048, 4 096 (5.8)
 //   40 words 16 x 3: 4.37, 5.13, 7.72 ms at 512, 2 048, 4 096 (10.8)
@@ -73,7 +74,10 @@ uint32_t pick_limbs(uint32_t words) { return pick_layout(32 * words, 0); }
 //            8 x 12: 27.5, 27.5, 39.7, 39.7
 //  135 words 16 x 9: 45.8, 66.9, 101.2 ms at 1 184, 2 368, 3 072
 //            8 x 17: 70.8, 70.8, 101.6
-// (16 words: 0.85 ms on one thread, 1.27 in groups).
+// Base 2 alone is doubled, so one thread per number keeps the sizes that its
+// kernel fills and a group pads: 16 words (0.85 ms, 1.27 in groups), 17 to 20
+// (17 words: 1.31 to 1.38 ms at 64 to 4 096 tests, 1.35 to 1.51 on 8 x 3; 20: 1.48 to
+// 1.56, 1.52 to 1.71) and 24 (2.50 to 2.57 ms at 64 to 1 536, 2.77 to 3.23 on 16 x 3).
 uint32_t pick_batch(uint32_t words, uint32_t n, uint32_t rounds, bool *side_by_side) {
     const uint32_t L = pick_limbs(words);
     *side_by_side = false;
@@ -87,8 +91,9 @@ uint32_t pick_batch(uint32_t words, uint32_t n, uint32_t rounds, bool *side_by_s
     }
     *side_by_side = rounds > 1 && n <= 1024;
     const uint32_t tests = *side_by_side ? 16 * n : n;
-    if (words > 16 && words <= 23 && tests <= 4096) return PG_LAYOUT_GROUP(8, 24);
-    if (words > 23 && words <= 47 && tests <= 64 * words) return PG_LAYOUT_GROUP(16, 48);
+    const bool base2 = !*side_by_side;
+    if (words > (base2 ? 20 : 16) && words <= 23 && tests <= 4096) return PG_LAYOUT_GROUP(8, 24);
+    if (words > (base2 ? 24 : 23) && words <= 47 && tests <= 64 * words) return PG_LAYOUT_GROUP(16, 48);
     if (words == 48 && tests <= 4096) return PG_LAYOUT_GROUP(8, 64);
     return L;
 }

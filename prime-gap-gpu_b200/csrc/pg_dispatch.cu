@@ -74,10 +74,15 @@ uint32_t pick_limbs(uint32_t words) { return pick_layout(32 * words, 0); }
 //            8 x 12: 27.5, 27.5, 39.7, 39.7
 //  135 words 16 x 9: 45.8, 66.9, 101.2 ms at 1 184, 2 368, 3 072
 //            8 x 17: 70.8, 70.8, 101.6
-// Base 2 alone is doubled, so one thread per number keeps the sizes that its
-// kernel fills and a group pads: 16 words (0.85 ms, 1.27 in groups), 17 to 20
-// (17 words: 1.31 to 1.38 ms at 64 to 4 096 tests, 1.35 to 1.51 on 8 x 3; 20: 1.48 to
-// 1.56, 1.52 to 1.71) and 24 (2.50 to 2.57 ms at 64 to 1 536, 2.77 to 3.23 on 16 x 3).
+// Other bases than 2 multiply where base 2 is doubled, which groups fold into
+// the squaring, so side by side they start at 17 words (64 primes, 16 bases: 17
+// words 1.4 ms, 26 in turn).  17 to 20 and 24 words stop where base 2 has no warp
+// of its own per number any more (launch_prp_bases_t), from where a batch of
+// composites would take longer than on one thread.  Base 2 alone keeps to one
+// thread per number at the sizes that its kernel fills and a group pads: 16 words
+// (0.85 ms, 1.27 in groups), 17 to 20 (17 words: 1.31 to 1.38 ms at 64 to 4 096
+// tests, 1.35 to 1.51 on 8 x 3; 20: 1.48 to 1.56, 1.52 to 1.71) and 24 (2.50 to 2.57 ms
+// at 64 to 1 536, 2.77 to 3.23 on 16 x 3).
 uint32_t pick_batch(uint32_t words, uint32_t n, uint32_t rounds, bool *side_by_side) {
     const uint32_t L = pick_limbs(words);
     *side_by_side = false;
@@ -91,9 +96,10 @@ uint32_t pick_batch(uint32_t words, uint32_t n, uint32_t rounds, bool *side_by_s
     }
     *side_by_side = rounds > 1 && n <= 1024;
     const uint32_t tests = *side_by_side ? 16 * n : n;
-    const bool base2 = !*side_by_side;
-    if (words > (base2 ? 20 : 16) && words <= 23 && tests <= 4096) return PG_LAYOUT_GROUP(8, 24);
-    if (words > (base2 ? 24 : 23) && words <= 47 && tests <= 64 * words) return PG_LAYOUT_GROUP(16, 48);
+    // lanes of base 2 at a warp per number, the other bases in groups of T lanes
+    const auto apart = [&](uint32_t T) { return *side_by_side && n * (32 + (rounds - 1) * T) <= 18944; };
+    if (words > 16 && words <= 23 && (words > 20 ? tests <= 4096 : apart(8))) return PG_LAYOUT_GROUP(8, 24);
+    if (words > 23 && words <= 47 && (words > 24 ? tests <= 64 * words : apart(16))) return PG_LAYOUT_GROUP(16, 48);
     if (words == 48 && tests <= 4096) return PG_LAYOUT_GROUP(8, 64);
     return L;
 }
@@ -103,13 +109,33 @@ uint32_t layout_words(uint32_t layout) { return layout & 0xffffu; }
 cudaError_t launch_prp_batch(uint32_t L, const uint32_t *cand, uint32_t words, uint32_t n, uint32_t rounds,
                              int32_t *out, bool side_by_side, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-#define PG_CASE(nl) \
-    if (L == nl) return launch_prp_batch_t<nl>(cand, words, n, rounds, out, side_by_side, st);
+    // Base 2 first, in a launch of its own and in the layout of a batch of it alone,
+    // where it would wait for the other bases: the code of base 2 and that of the
+    // others, each too long for the instruction cache, slow each other down.  One
+    // thread per number from 25 words on: from a warp an SM (1 024 composites, 16
+    // bases: 32 words 5.7 ms in turn, 6.6 side by side, 40 words 10.9 and 14.8; at 48
+    // words the two spill); the widest groups: from two (74 composites of 144 words
+    // 101.8 and 109.9 ms).  The others run beside it as fast as after it.
+    const uint32_t lanes = L >> 16 ? L >> 16 : 1, warps = n * ((rounds - 1) * lanes + (lanes > 1 ? 32 : 1)) / 32;
+    const bool tested = side_by_side && (L == 48 || (L >= 28 && lanes == 1 && warps > 148) ||
+                                         (L == PG_LAYOUT_GROUP(8, 160) && warps > 2 * 148));
+    if (tested) {
+        bool one = false;
+        const cudaError_t e = launch_prp_batch(pick_batch(words, n, 1, &one), cand, words, n, 1, out, one, st);
+        if (e != cudaSuccess) return e;
+    }
+#define PG_CASE(nl)                                                                                              \
+    if (L == nl)                                                                                                 \
+        return side_by_side                                                                                      \
+                   ? launch_prp_bases_t<OneThread<nl>>(cand, words, n, rounds, out, tested, st)                  \
+                   : launch_prp_batch_t<nl>(cand, words, n, rounds, out, st);
     PG_LIMB_LIST(PG_CASE)
 #undef PG_CASE
-#define PG_GCASE(t, lt) \
-    if (L == PG_LAYOUT_GROUP(t, (t) * (lt)))            \
-        return glaunch_prp_batch<t, lt>(cand, words, n, rounds, out, side_by_side, st);
+#define PG_GCASE(t, lt)                                                                                              \
+    if (L == PG_LAYOUT_GROUP(t, (t) * (lt)))                                                                         \
+        return side_by_side                                                                                          \
+                   ? launch_prp_bases_t<LaneGroup<t, lt>>(cand, words, n, rounds, out, tested, st)                    \
+                   : glaunch_prp_batch<t, lt>(cand, words, n, rounds, out, st);
     PG_GROUP_LIST(PG_GCASE)
 #undef PG_GCASE
     return cudaErrorInvalidValue;

@@ -286,8 +286,9 @@ __device__ __forceinline__ void gdbl(const Group<T> &G, uint32_t (&x)[LT], const
 
 // Strong probable-prime test of the odd group-held n (> base + 1) to `base`
 // (miller_rabin.h:216-248 for one base).  bits(n) <= 32*L - 2 is required.
-template <int T, int LT, bool FOLD = false>
-__device__ __forceinline__ bool gstrong_prp(const Group<T> &G, const uint32_t (&n)[LT], uint32_t base) {
+template <int T, int LT, bool FOLD = false, class Over = NeverOver>
+__device__ __forceinline__ bool gstrong_prp(const Group<T> &G, const uint32_t (&n)[LT], uint32_t base,
+                                            const Over &ov = Over()) {
     // ninv from the lowest word (lane 0), B and s = ctz(n-1) over the group
     const uint32_t n0 = __shfl_sync(G.gmask, n[0], G.gb);
     const uint32_t ninv = neg_inv32(n0);
@@ -366,6 +367,7 @@ __device__ __forceinline__ bool gstrong_prp(const Group<T> &G, const uint32_t (&
 #pragma unroll
     for (int k = 0; k < LT; k++) nm1[k] = (G.gl == 0 && k == 0) ? (n[0] & ~1u) : n[k];
     for (int b = fold ? B - 1 : B - 2;; b--) {
+        const int32_t seen = ov.peek();
         if (b < s) {
             uint32_t y[LT];
             gmont_mul<T, LT>(G, y, x, unit, n, ninv);  // leave Montgomery form: y in [0, n]
@@ -395,6 +397,8 @@ __device__ __forceinline__ bool gstrong_prp(const Group<T> &G, const uint32_t (&
             else
                 gmont_mul<T, LT>(G, x, x, bm, n, ninv);
         }
+        // lane 0's reading for the whole group: the lanes stay together
+        if (Over::may && ov.over(__shfl_sync(G.gmask, seen, G.gb))) return true;
     }
 }
 

@@ -235,6 +235,7 @@ cudaError_t launch_confirm(uint32_t L, const SearchArgs &a, uint32_t *gaps, uint
                            uint32_t *n_redo, unsigned long long *confirm_tests, uint32_t *k_start_rw,
                            cudaStream_t st);
 cudaError_t launch_iota(uint32_t *out, uint32_t n, cudaStream_t st);
+cudaError_t launch_set(int32_t *out, uint32_t n, int32_t f, int32_t v, cudaStream_t st);  // out = f * out + v
 // found_k = NOT_FOUND, k_start = 0, act = 0..S-1, conf = NOT_FOUND for S
 // sides; the scalars' queue head and counters = 0, unresolved = S,
 // active_warps = warps

@@ -1191,6 +1191,18 @@ __global__ void k_iota(uint32_t *out, uint32_t n) {
     if (i < n) out[i] = i;
 }
 
+// out[i] = f * out[i] + v, without reading out where f is 0
+__global__ void k_set(int32_t *out, uint32_t n, int32_t f, int32_t v) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = f ? f * out[i] + v : v;
+}
+
+cudaError_t launch_set(int32_t *out, uint32_t n, int32_t f, int32_t v, cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    k_set<<<(n + 255) / 256, 256, 0, st>>>(out, n, f, v);
+    return cudaGetLastError();
+}
+
 __global__ void k_init_search(uint32_t S, uint32_t *found_k, uint32_t *k_start, uint32_t *act, uint32_t *conf,
                               Scalars *sc, uint32_t warps) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -308,13 +308,31 @@ __device__ __forceinline__ int bit_length(const uint32_t (&n)[L]) {
     return b;
 }
 
+// When a test may be given up: never, or once the number has failed an
+// earlier base than the r-th (the bases of a number side by side; *first = the
+// earliest base known to fail).  peek() reads, over() judges what was read, so
+// the read's latency passes under a step.
+struct NeverOver {
+    static constexpr bool may = false;
+    __device__ __forceinline__ int32_t peek() const { return 0; }
+    __device__ __forceinline__ bool over(int32_t) const { return false; }
+};
+struct OverByBase {
+    static constexpr bool may = true;
+    const int32_t *first;
+    int32_t r;
+    __device__ __forceinline__ int32_t peek() const { return *(const volatile int32_t *)first; }
+    __device__ __forceinline__ bool over(int32_t seen) const { return seen < r; }
+};
+
 // Strong probable-prime test of odd n > base+1 to the given base
-// (miller_rabin.h:216-248 for one base).  Returns true if n passes.
+// (miller_rabin.h:216-248 for one base).  Returns true if n passes (or the
+// test was given up).
 // One loop walks the bits of n-1 from the top: above bit s it squares and
 // multiplies by the base; from bit s-1 down it is the squaring chain of the
 // strong test, checked against 1 and n-1 after leaving Montgomery form.
-template <int L>
-__device__ __forceinline__ bool strong_prp(const uint32_t (&n)[L], uint32_t base) {
+template <int L, class Over = NeverOver>
+__device__ __forceinline__ bool strong_prp(const uint32_t (&n)[L], uint32_t base, const Over &ov = Over()) {
     const uint32_t ninv = neg_inv32(n[0]);
     const int B = bit_length<L>(n);
     // s = ctz(n - 1); n is odd so n - 1 = n with bit 0 cleared
@@ -347,6 +365,7 @@ __device__ __forceinline__ bool strong_prp(const uint32_t (&n)[L], uint32_t base
 #pragma unroll
     for (int k = 0; k < L; k++) e[k] = n[k];
     for (int b = B - 2;; b--) {
+        const int32_t seen = ov.peek();
         if (b < s) {
             uint32_t t[2 * L + 1];
 #pragma unroll
@@ -370,6 +389,7 @@ __device__ __forceinline__ bool strong_prp(const uint32_t (&n)[L], uint32_t base
             else
                 mod_mul_small<L>(x, n, base);
         }
+        if (ov.over(seen)) return true;
     }
 }
 

@@ -1,6 +1,7 @@
 // pg_search.cuh -- PRP kernels templated on the limb count L.
 //
 //   k_prp_batch          strong PRP of a batch (miller_rabin.h:252-270)
+//   k_prp_bases          the same with the bases of a number side by side
 //   k_search_persistent  persistent PRP search with a device work queue
 //                        (replaces gpu_testing.cu:203-350 and the CPU overflow
 //                        threads of overflow.cpp:61-227)
@@ -36,28 +37,63 @@ __global__ void __launch_bounds__(128) k_prp_batch(const uint32_t *__restrict__ 
     out[i] = prp_rounds<L>(x, (int)rounds);
 }
 
-// The bases of one number side by side, 16 lanes a number: for batches so
-// small that the bases in turn would leave the device idle (12 numbers of 22
-// words, 16 bases: 48 ms in turn, 2 ms side by side).
+// The bases of a number side by side, for batches so small that the bases in
+// turn would leave the device idle (12 numbers of 22 words, 16 bases: 48 ms in
+// turn, 1.7 ms side by side).  out[i] = first base that fails, set to `rounds`
+// before.  One-warp blocks: the first `scouts` blocks test base 2, the others
+// bases 3, 5, ..., and give up once an earlier base has failed.  Base 2 keeps to warps of its own because it is the cheapest
+// (doublings) and alone decides nearly every composite: a batch without a
+// prime takes the time of base 2, as with the bases in turn (64 numbers, 16
+// bases: 16 words 0.75 ms, 0.75 in turn, 1.84 with a number's bases in one warp; 64
+// words 12.4, 18.9, 17.9; all prime: 0.53 and 8.4 ms, 4.9 and 358 in turn).
 template <int L>
-__global__ void __launch_bounds__(128) k_prp_bases(const uint32_t *__restrict__ cand, uint32_t words, uint32_t n,
-                                                   uint32_t rounds, int32_t *__restrict__ out) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> 4, r = t & 15;
-    bool fail = false;
-    if (i < n && r < rounds) {
+struct OneThread {
+    static constexpr int lanes = 1;
+    template <class Over>
+    static __device__ __forceinline__ bool fails(const uint32_t *__restrict__ row, uint32_t words, uint32_t r,
+                                                 const Over &ov) {
         uint32_t x[L];
         uint32_t hi = 0;
 #pragma unroll
-        for (int k = 0; k < L; k++) x[k] = ((uint32_t)k < words) ? cand[(size_t)i * words + k] : 0u;
+        for (int k = 0; k < L; k++) x[k] = ((uint32_t)k < words) ? row[k] : 0u;
 #pragma unroll
         for (int k = 1; k < L; k++) hi |= x[k];
-        if ((x[0] & 1u) == 0 || (hi == 0 && x[0] < 3))
-            fail = true;
-        else
-            fail = !tiny_pass<L>(x, prp_base(r)) && !strong_prp<L>(x, prp_base(r));
+        if ((x[0] & 1u) == 0 || (hi == 0 && x[0] < 3)) return r == 0;
+        if (ov.over(ov.peek())) return false;
+        const uint32_t base = Over::may ? prp_base(r) : 2u;
+        return !tiny_pass<L>(x, base) && !strong_prp<L>(x, base, ov);
     }
-    const unsigned bad = (__ballot_sync(0xffffffffu, fail) >> (threadIdx.x & 16)) & 0xffffu;
-    if (i < n && r == 0) out[i] = bad ? __ffs(bad) - 1 : (int)rounds;
+};
+
+template <class N>
+__global__ void __launch_bounds__(32) k_prp_bases(const uint32_t *__restrict__ cand, uint32_t words, uint32_t n,
+                                                  uint32_t rounds, uint32_t scouts, uint32_t per_scout, int32_t *out) {
+    const uint32_t slot = threadIdx.x / N::lanes;
+    if (blockIdx.x < scouts) {
+        const uint32_t i = blockIdx.x * per_scout + slot;
+        if (slot < per_scout && i < n && N::fails(cand + (size_t)i * words, words, 0, NeverOver())) atomicMin(&out[i], 0);
+    } else {
+        const uint32_t t = (blockIdx.x - scouts) * (32 / N::lanes) + slot;
+        const uint32_t i = t / (rounds - 1), r = 1 + t % (rounds - 1);
+        if (i < n && N::fails(cand + (size_t)i * words, words, r, OverByBase{out + i, (int32_t)r}))
+            atomicMin(&out[i], (int32_t)r);
+    }
+}
+
+// tested: out holds the verdicts of base 2 already (1 = passed).  Groups that
+// test base 2 take a warp each while all warps have an SM quarter of their own:
+// the groups of a warp step through different numbers, and each waits for the
+// doublings of the others (22 words 1.38 ms alone in a warp, 1.61 four to a warp).
+template <class N>
+cudaError_t launch_prp_bases_t(const uint32_t *cand, uint32_t words, uint32_t n, uint32_t rounds, int32_t *out,
+                               bool tested, cudaStream_t st) {
+    const cudaError_t e = tested ? launch_set(out, n, (int32_t)rounds, 0, st) : launch_set(out, n, 0, (int32_t)rounds, st);
+    if (e != cudaSuccess) return e;
+    const uint32_t others = (n * (rounds - 1) * N::lanes + 31) / 32;
+    const uint32_t per_scout = N::lanes > 1 && n + others <= 4 * 148 ? 1 : 32 / N::lanes;
+    const uint32_t scouts = tested ? 0 : (n + per_scout - 1) / per_scout;
+    k_prp_bases<N><<<scouts + others, 32, 0, st>>>(cand, words, n, rounds, scouts, per_scout, out);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------ search core
@@ -357,11 +393,7 @@ __global__ void __launch_bounds__(128) k_confirm(const __grid_constant__ SearchA
 
 template <int L>
 cudaError_t launch_prp_batch_t(const uint32_t *cand, uint32_t words, uint32_t n, uint32_t rounds, int32_t *out,
-                               bool side_by_side, cudaStream_t st) {
-    if (side_by_side) {
-        k_prp_bases<L><<<(n + 7) / 8, 128, 0, st>>>(cand, words, n, rounds, out);
-        return cudaGetLastError();
-    }
+                               cudaStream_t st) {
     const uint32_t threads = 128, blocks = (n + threads - 1) / threads;
     k_prp_batch<L><<<blocks, threads, 0, st>>>(cand, words, n, rounds, out);
     return cudaGetLastError();
@@ -406,7 +438,9 @@ cudaError_t launch_confirm_t(const SearchArgs &a, uint32_t *gaps, uint32_t *conf
 
 #define PG_DECLARE_LIMBS(L)                                                                                       \
     extern template cudaError_t launch_prp_batch_t<L>(const uint32_t *, uint32_t, uint32_t, uint32_t, int32_t *,  \
-                                                      bool, cudaStream_t);                                        \
+                                                      cudaStream_t);                                              \
+    extern template cudaError_t launch_prp_bases_t<OneThread<L>>(                                                 \
+        const uint32_t *, uint32_t, uint32_t, uint32_t, int32_t *, bool, cudaStream_t);                           \
     extern template int search_occupancy_t<L>();                                                                  \
     extern template cudaError_t launch_search_persistent_t<L>(const SearchArgs &, int, cudaStream_t);            \
     extern template cudaError_t launch_search_plain_t<L>(const SearchArgs &, uint32_t *, cudaStream_t);          \
@@ -416,8 +450,10 @@ cudaError_t launch_confirm_t(const SearchArgs &a, uint32_t *gaps, uint32_t *conf
                                                     uint32_t *, unsigned long long *, uint32_t *, cudaStream_t);
 
 #define PG_INSTANTIATE_LIMBS(L)                                                                                   \
-    template cudaError_t launch_prp_batch_t<L>(const uint32_t *, uint32_t, uint32_t, uint32_t, int32_t *, bool,   \
+    template cudaError_t launch_prp_batch_t<L>(const uint32_t *, uint32_t, uint32_t, uint32_t, int32_t *,         \
                                                cudaStream_t);                                                     \
+    template cudaError_t launch_prp_bases_t<OneThread<L>>(const uint32_t *, uint32_t, uint32_t, uint32_t,         \
+                                                          int32_t *, bool, cudaStream_t);                         \
     template int search_occupancy_t<L>();                                                                         \
     template cudaError_t launch_search_persistent_t<L>(const SearchArgs &, int, cudaStream_t);                   \
     template cudaError_t launch_search_plain_t<L>(const SearchArgs &, uint32_t *, cudaStream_t);                 \

@@ -80,34 +80,29 @@ __global__ void __launch_bounds__(128) k_prp_batch_g(const uint32_t *__restrict_
     if (G.gl == 0) out[i] = passed;
 }
 
-// The bases of one number side by side (k_prp_bases): a block of 16 groups
-// takes one number.
+// One number on a group of lanes, for k_prp_bases.
 template <int T, int LT>
-__global__ void __launch_bounds__(16 * T) k_prp_bases_g(const uint32_t *__restrict__ cand, uint32_t words, uint32_t n,
-                                                        uint32_t rounds, int32_t *__restrict__ out) {
-    __shared__ uint32_t s_bad;
-    const Group<T> G;
-    const uint32_t i = blockIdx.x, r = threadIdx.x / T;
-    if (threadIdx.x == 0) s_bad = 0;
-    __syncthreads();
-    if (r < rounds) {
+struct LaneGroup {
+    static constexpr int lanes = T;
+    template <class Over>
+    static __device__ __forceinline__ bool fails(const uint32_t *__restrict__ row, uint32_t words, uint32_t r,
+                                                 const Over &ov) {
+        const Group<T> G;
         uint32_t x[LT];
         uint32_t hi = 0;
 #pragma unroll
         for (int k = 0; k < LT; k++) {
             const uint32_t wi = G.gl * LT + k;
-            x[k] = wi < words ? cand[(size_t)i * words + wi] : 0u;
+            x[k] = wi < words ? row[wi] : 0u;
             hi |= wi ? x[k] : 0u;
         }
         const bool big = G.field(__ballot_sync(G.gmask, hi != 0)) != 0;
-        const uint32_t n0 = __shfl_sync(G.gmask, x[0], G.gb), base = prp_base(r);
-        bool fail = (n0 & 1u) == 0 || (!big && n0 < 3);
-        if (!fail && (big || n0 - 1 > base)) fail = !gstrong_prp<T, LT, true>(G, x, base);
-        if (fail && G.gl == 0) atomicOr(&s_bad, 1u << r);
+        const uint32_t n0 = __shfl_sync(G.gmask, x[0], G.gb);
+        const uint32_t base = Over::may ? prp_base(r) : 2u;
+        if ((n0 & 1u) == 0 || (!big && n0 < 3)) return r == 0;
+        return (big || n0 - 1 > base) && !gstrong_prp<T, LT, Over::may>(G, x, base, ov);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) out[i] = s_bad ? __ffs(s_bad) - 1 : (int)rounds;
-}
+};
 
 // Persistent search with one item per group (see k_search_persistent).
 template <int T, int LT>
@@ -302,11 +297,7 @@ __global__ void __launch_bounds__(128) k_confirm_g(const __grid_constant__ Searc
 
 template <int T, int LT>
 cudaError_t glaunch_prp_batch(const uint32_t *cand, uint32_t words, uint32_t n, uint32_t rounds, int32_t *out,
-                              bool side_by_side, cudaStream_t st) {
-    if (side_by_side) {
-        k_prp_bases_g<T, LT><<<n, 16 * T, 0, st>>>(cand, words, n, rounds, out);
-        return cudaGetLastError();
-    }
+                              cudaStream_t st) {
     const uint64_t threads = (uint64_t)n * T;
     k_prp_batch_g<T, LT><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(cand, words, n, rounds, out);
     return cudaGetLastError();
@@ -352,7 +343,9 @@ cudaError_t glaunch_confirm(const SearchArgs &a, uint32_t *gaps, uint32_t *conf,
 
 #define PG_GDECLARE(T, LT)                                                                                        \
     extern template cudaError_t glaunch_prp_batch<T, LT>(const uint32_t *, uint32_t, uint32_t, uint32_t,         \
-                                                         int32_t *, bool, cudaStream_t);                         \
+                                                         int32_t *, cudaStream_t);                               \
+    extern template cudaError_t launch_prp_bases_t<LaneGroup<T, LT>>(                                             \
+        const uint32_t *, uint32_t, uint32_t, uint32_t, int32_t *, bool, cudaStream_t);                           \
     extern template int gsearch_occupancy<T, LT>();                                                               \
     extern template cudaError_t glaunch_search_persistent<T, LT>(const SearchArgs &, int, cudaStream_t);         \
     extern template cudaError_t glaunch_search_plain<T, LT>(const SearchArgs &, uint32_t *, cudaStream_t);       \
@@ -363,7 +356,9 @@ cudaError_t glaunch_confirm(const SearchArgs &a, uint32_t *gaps, uint32_t *conf,
 
 #define PG_GINSTANTIATE(T, LT)                                                                                    \
     template cudaError_t glaunch_prp_batch<T, LT>(const uint32_t *, uint32_t, uint32_t, uint32_t, int32_t *,     \
-                                                  bool, cudaStream_t);                                            \
+                                                  cudaStream_t);                                                  \
+    template cudaError_t launch_prp_bases_t<LaneGroup<T, LT>>(                                                    \
+        const uint32_t *, uint32_t, uint32_t, uint32_t, int32_t *, bool, cudaStream_t);                           \
     template int gsearch_occupancy<T, LT>();                                                                      \
     template cudaError_t glaunch_search_persistent<T, LT>(const SearchArgs &, int, cudaStream_t);                \
     template cudaError_t glaunch_search_plain<T, LT>(const SearchArgs &, uint32_t *, cudaStream_t);              \

@@ -28,3 +28,9 @@ def test_sizes_that_one_thread_fills_stay_on_one_thread(pg, words, layout, n):
                                             (48, 4096, _group(8, 64)), (48, 4097, 48)])
 def test_few_longer_numbers_take_groups(pg, words, n, layout):
     assert _layout(pg, words, n) == layout
+
+
+@pytest.mark.parametrize("words,n,layout", [(16, 1024, 16), (17, 124, _group(8, 24)), (20, 125, 20), (23, 256, _group(8, 24)),
+                                            (24, 69, _group(16, 48)), (24, 70, 24), (25, 100, _group(16, 48))])
+def test_layouts_of_bases_side_by_side(pg, words, n, layout):
+    assert _layout(pg, words, n, 16) == layout

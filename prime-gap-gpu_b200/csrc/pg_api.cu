@@ -768,12 +768,14 @@ static uint64_t seg_bands(const pg_job *j, uint64_t split, uint64_t nodd, SegBan
     return hi;
 }
 
-// First prime-table index sieved by the primes' lattices: those expecting at
-// most LAT_HITS hits in the window; none for a job that forces the search.
-static uint64_t lattice_first(const pg_job *j, uint64_t m0, uint64_t nodd) {
+// First prime-table index sieved by the primes' lattices in a window of nodd odd
+// m: those expecting at most LAT_HITS hits, none where they are few (LAT_FEW) or
+// the job forces the search.
+static uint64_t lattice_cut(const pg_job *j, uint64_t nodd) {
     const pg::Tables &T = *j->T;
-    if (!T.lat || (j->prm.flags & PG_JOB_LARGE_SEARCH) || m0 >= (1ull << 30) || nodd >= (1ull << 30)) return T.np;
-    return table_index_at(T, (double)nodd * (2.0 * j->sly + 1) / LAT_HITS);
+    if (!T.lat || (j->prm.flags & PG_JOB_LARGE_SEARCH)) return T.np;
+    const uint64_t cut = table_index_at(T, (double)nodd * (2.0 * j->sly + 1) / LAT_HITS);
+    return T.np - cut < LAT_FEW && cut > table_index_at(T, 2.0 * j->sly + 2) ? T.np : cut;
 }
 
 // sieve of one window of the slot into its rows of lists (compact) or into
@@ -802,7 +804,8 @@ static int run_sieve(Slot &s, const WinPart &w, bool compact) {
     SegBand bands[MAX_SEG_BANDS];
     int nb = 0;
     const uint64_t search_first = seg_bands(j, split, w.nodd, bands, &nb);
-    const uint64_t lat_first = std::max(search_first, lattice_first(j, w.m0, w.nodd));
+    const bool in_range = w.m0 < (1ull << 30) && w.nodd < (1ull << 30);  // of lattice_hits' 32-bit values
+    const uint64_t lat_first = in_range ? std::max(search_first, lattice_cut(j, w.nodd)) : T.np;
     la.lat = lat_first < T.np ? T.lat.load() : nullptr;
     PG_CUDA(launch_sieve_large(la, T.wide, split, bands, nb, search_first, lat_first, s.st));
     s.sst.kernel_launches += (split > 0) + (nb > 0) + (search_first < lat_first) + (lat_first < T.np);
@@ -1317,14 +1320,14 @@ static int job_build(pg_job *j) {
     if (2 * j->nm_cap >= 0xffffffffull) return fail(PG_ERR_UNSUPPORTED, "max_m_inc too large");
     // ---- walk steps of the large primes below 2^32 for this job's window width
     // (with PG_JOB_COMPACT_WALK only of those expecting >= SEG_HITS hits in the
-    // largest window, which the segmented kernel needs; the lattices find the
-    // hits of those expecting at most LAT_HITS)
+    // largest window, which the segmented kernel needs; without it not of those
+    // that the largest window leaves to the lattices)
     if (T.np && !(p.flags & PG_JOB_LARGE_STEP)) {
         const uint64_t first = table_index_at(T, 2.0 * j->sly + 2);
         double pmax = 4294967296.0;
         if (p.flags & PG_JOB_COMPACT_WALK)
             pmax = (double)j->nodd_cap * (2.0 * j->sly + 1) / SEG_HITS;
-        else if (T.lat && !(p.flags & PG_JOB_LARGE_SEARCH) && p.max_m < (1ull << 30))
+        else if (p.max_m < (1ull << 30) && lattice_cut(j, j->nodd_cap) < T.np)
             pmax = (double)j->nodd_cap * (2.0 * j->sly + 1) / LAT_HITS;
         // table_index_at keeps the whole segment holding pmax: with primes above
         // 2^32 in the table, stop a segment early so every kept prime is below 2^32

@@ -179,7 +179,13 @@ constexpr uint32_t LAT_W = 1u << 13;
 // so every prime below 2^36 qualifies; the others' are kept out.
 constexpr uint32_t LAT_MAX_M = 1u << 24;
 constexpr double LAT_EDGE = 1e-4;
+// Lattices sieve the primes that expect at most LAT_HITS hits, unless that
+// takes a second launch for fewer than LAT_FEW of them: its ramp and tail cost
+// what 2 million searches do (sieve of P = 337, primes <= 1e8: 14 000 m, 2.6 million
+// primes, 0.37 ms and 0.38 without; 20 000 m, 1.4 million, 0.50 and 0.49; sl 2 000,
+// 4 000 m, primes <= 2e7, 1 million, 0.16 and 0.12).
 constexpr double LAT_HITS = 1.0;
+constexpr uint64_t LAT_FEW = 1ull << 21;
 
 // Primes of the large-prime table processed by the segmented kernel in one
 // launch: [first, first + count), each split into nseg segments of seg_len

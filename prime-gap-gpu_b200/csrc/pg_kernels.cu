@@ -722,10 +722,34 @@ __device__ __forceinline__ void lattice_hits(const LargeArgs &a, const uint32_t 
         x -= M;
     }
     int64_t u = (int64_t)b - ((int64_t)t * l.dec + (int64_t)Q * l.w);  // b - S
+    if (M >= J) {  // at most one point a row
+        while (true) {
+            if (x < J && (uint64_t)u <= W) mark_hit(a, s_wheel, (uint64_t)x, (uint32_t)u);
+            if (--t < t0) return;
+            x += (int32_t)l.inc;
+            u += l.dec;
+            if (x >= M) {
+                x -= M;
+                u += l.w;
+            }
+        }
+    }
+    // The points of a row are M apart in x and w apart in S: those within [0, W]
+    // follow one another.  A row is entered one or two points before them, so a
+    // prime with a short M costs its hits and not its rows (its J / M points
+    // had sent it to the modular search, a lane of nearly every warp at small sl:
+    // P = 337, sl 2 000, 10 000 m, primes <= 2e7: sieve 0.27 -> 0.21 ms).
+    const double rw = fast_rcp((double)l.w);
+    const int64_t enter = l.w > 0 ? (int64_t)W : 0;
     while (true) {
-        int64_t v = u;
-        for (int32_t y = x; y < J; y += M, v -= l.w)
-            if ((uint64_t)v <= W) mark_hit(a, s_wheel, (uint64_t)y, (uint32_t)v);
+        const int32_t skip = (uint64_t)u <= W ? 0 : max(__double2int_rd((double)(u - enter) * rw) - 1, 0);
+        int64_t v = u - (int64_t)skip * l.w;
+        for (int32_t y = skip <= (J - 1 - x) / M ? x + skip * M : J; y < J; y += M, v -= l.w) {
+            if ((uint64_t)v <= W)
+                mark_hit(a, s_wheel, (uint64_t)y, (uint32_t)v);
+            else if (l.w > 0 ? v < 0 : v > (int64_t)W)
+                break;
+        }
         if (--t < t0) return;
         x += (int32_t)l.inc;
         u += l.dec;
@@ -867,14 +891,13 @@ cudaError_t launch_lattices(const void *p, const void *c, const void *ci, bool w
 }
 
 // The primes [first, first + count) by their lattices, one thread each; the
-// few without one (or with so short a step that a row of x would be long) by
-// modular search.  Reads each prime's p, K mod p and lattice (24 or 32 B) once:
-// 2.7 TB/s at 32-bit primes and 3.1 TB/s at 64-bit ones, with the integer
-// pipe half busy and the conversions 40 %.  Where primes expect at most one
-// hit it replaces ten Euclid levels a prime (P = 907, 20 000 m, primes <= 1e10:
-// sieve 16.5 -> 6.0 ms; P = 503, 1 500 m, primes <= 1e9: 1.20 -> 0.49); with
+// few without one by modular search.  Reads each prime's p, K mod p and lattice
+// (24 or 32 B) once: 2.8 TB/s at 32-bit primes and 3.2 TB/s at 64-bit ones, with
+// the integer pipe half busy and the conversions 40 %.  Where primes expect at
+// most one hit it replaces ten Euclid levels a prime (P = 907, 20 000 m, primes
+// <= 1e10: sieve 16.5 -> 5.2 ms; P = 503, 1 500 m, primes <= 1e9: 1.20 -> 0.48); with
 // more hits the lanes of a warp wait for the longest enumeration and the
-// search with its walk is the faster (P = 503, 200 000 m: 5.45 ms with the
+// search with its walk is the faster (P = 503, 200 000 m: 5.15 ms with the
 // line at 1 hit, 7.2 at 4 hits, 5.7 without lattices).
 template <typename T, bool F>
 __global__ void __launch_bounds__(256, 6) k_sieve_large_lattice(const __grid_constant__ LargeArgs a, uint64_t first,
@@ -886,7 +909,7 @@ __global__ void __launch_bounds__(256, 6) k_sieve_large_lattice(const __grid_con
     if (i >= first + count) return;
     const LatC l = a.lat[i];
     const T p = ((const T *)a.p)[i], c = ((const T *)a.c)[i];
-    if (l.M && (uint64_t)l.M * 64 >= a.nodd) {
+    if (l.M) {
         lattice_hits<T>(a, s_wheel, p, c, l);
         return;
     }

@@ -6,7 +6,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-ARGS = dict(p=337, d=2310, sl=3_000, max_prime=20_000_000, max_m_inc=4_000, max_m=11_000_000)
+ARGS = dict(p=337, d=2310, sl=3_000, max_prime=100_000_000, max_m_inc=4_000, max_m=11_000_000)
 
 
 def test_large_search_flag_forces_the_search(pg):

@@ -994,6 +994,16 @@ int pg::slot_resume(Slot &s) {
     return enqueue_finalize(s, a, S);
 }
 
+// How much longer a round takes for each further warp on an SM quarter with LT
+// words on each of T lanes: fewer words and fewer shuffles of a row leave more
+// latency that another warp fills.  Fitted to rounds of full searches at 4 and 12
+// warps per SM: 4 x 6 0.18 a warp, 4 x 12 0.37, 8 x 3 0.14, 8 x 8 0.40, 8 x 17 0.55,
+// 16 x 2 0.12, 16 x 6 0.43, 16 x 9 0.53.
+static double group_slope(uint32_t layout) {
+    const uint32_t T = layout >> 16, LT = layout_words(layout) / T;
+    return std::min(0.55, LT * (0.016 + 0.0033 * T));
+}
+
 // Blocks per SM of a search over the slot's sides.  Every block tests `per`
 // candidates at a time, the nearest of the sides still open, and c blocks on an
 // SM take 1 + slope (c - step) / step times as long per round as `step` of
@@ -1007,15 +1017,17 @@ int pg::slot_resume(Slot &s) {
 // ended have ended too, at most a quarter of its round (an eighth in searches
 // of more than 12 rounds, where the waits cost more than they save): 10 000 m
 // of P = 337 2.91 ms at an eighth, 2.58 at a quarter; 20 000 m of P = 907 74.2
-// without, 61.9 at either; 200 000 m of P = 503 69.1, 69.9 and 71.5.  A launch that shares the device
-// takes all blocks and never waits (15 mixed requests on a server: 201 ms with
-// the rule on every launch, 178 without).
+// without, 61.9 at either; 200 000 m of P = 503 69.1, 69.9 and 71.5.  A launch
+// that shares the device takes all blocks and never waits (15 mixed requests on a
+// server: 201 ms with the rule on every launch, 178 without).
 //   tensor-core kernel, per = 128, step 1, slope 0.33 (L = 15: 2 520, 3 520,
 //   4 090, 5 000 cycles a step at c = 1 .. 4), 0.43 (L = 23: 3 800, 4 940, 7 020,
 //   8 910) or 0.37 (L = 40: 8 020, 11 030 at c = 1, 2): 345 m of P = 503 4.98 ms at
 //   c = 4, 3.2 with the rule; 1 000 m of P = 907 15.7 and 12.1 ms
-//   lane groups, per = 32 / T, step 4, slope 0.57 (8 x 17: 70, 112, 150 ms a
-//   test at c = 4, 8, 12)
+//   lane groups, per = 32 / T, step 4, group_slope; with every block that fits
+//   they do not wait (900 000 tests of 1 295 bits on 8 x 8: 98 ms waiting, 94 not):
+//   600 m of P = 503 on 16 x 3 9.9 ms with the rule, 10.7 with all blocks, 13.9 at the
+//   slope of 8 x 17
 static int round_blocks(Slot &s, int most, int step, double slope, double per) {
     const int sms = s.parts[0].job->ctx->sms;
     double tests = 0, sides = 0;
@@ -1044,6 +1056,7 @@ static int round_blocks(Slot &s, int most, int step, double slope, double per) {
             s.settle = rounds <= 12 ? 16 : 8;
         }
     }
+    if (best == most && step > 1) s.settle = 0;
     return best;
 }
 
@@ -1078,7 +1091,7 @@ int pg::slot_enqueue(Slot &s, int form, uint32_t flags, bool graph) {
         else
             s.tc_grid = sms * (s.shared ? most : round_blocks(s, most, 1, s.tcL < 20 ? 0.33 : s.tcL < 30 ? 0.43 : 0.37, 128));
     } else if ((s.L >> 16) && !wps && !s.shared && form == PG_SEARCH_PERSISTENT && !(flags & PG_SUBMIT_DRAIN)) {
-        s.grid = sms * round_blocks(s, s.grid / sms, 4, 0.57, 32.0 / (s.L >> 16));
+        s.grid = sms * round_blocks(s, s.grid / sms, 4, group_slope(s.L), 32.0 / (s.L >> 16));
     }
     if (form == PG_SEARCH_PLAIN || !graph) return enqueue_windows(s, form, flags);
     // The persistent form's whole window (upload, sieves, search, finalize,

@@ -230,10 +230,27 @@ def kernel_products_per_test(bits: int, limbs: int) -> int:
 
 
 def tc_products_per_test(bits: int, limbs: int) -> int:
-    """32x32->64 limb products k_search_tc runs on the integer pipe per test: bits - 1 steps, each the square's
-    L(L+1)/2 cross and diagonal products and 2L for m*w - X*z; the reduction's two products are u8 matrices on
-    the tensor cores."""
-    return (bits - 1) * (limbs * (limbs + 1) // 2 + 2 * limbs)
+    """32x32->64 limb products k_search_tc runs on the integer pipe per test: a step for every bit of the exponent
+    that the start does not hold (tc_steps), each the square's L(L+1)/2 cross and diagonal products and 2L for
+    m*w - X*z; the reduction's two products are u8 matrices on the tensor cores."""
+    return tc_steps(bits, limbs) * (limbs * (limbs + 1) // 2 + 2 * limbs)
+
+
+def tc_steps(bits: int, limbs: int) -> int:
+    """Steps of a test of k_search_tc: below 40 words it starts from the exponent's leading floor(log2(bits - 32))
+    bits (pg_tc_search.cuh)."""
+    return bits - 1 - (0 if limbs >= 40 else (bits - 32).bit_length() - 1)
+
+
+def search_work(info: dict, bits: int, ran_tc: bool) -> tuple[str, int, str]:
+    """(kernel, limb products per test, what they are) of the persistent search that ran."""
+    if ran_tc:
+        L = info["tc_words"]
+        return (f"k_search_tc<{L}>", tc_products_per_test(bits, L),
+                f"{tc_steps(bits, L)} steps of {L} words: L(L+1)/2 + 2L each; the reduction is two u8 matrix products "
+                "on the tensor cores")
+    L, name = info["limbs"], "k_search_persistent" + ("" if info["tpi"] == 1 else "_g")
+    return f"{name}<{L}>", kernel_products_per_test(bits, L), f"{bits - 1} steps of {L} words: L(L+1)/2 + L^2 + L each"
 
 
 def traffic_per_launch() -> dict | None:
@@ -246,7 +263,7 @@ def traffic_per_launch() -> dict | None:
     return None
 
 
-HBM_FALLBACK_GBS = 6650.0  # an earlier copy-bandwidth measurement on this pool's B200s
+HBM_FALLBACK_GBS = 6650.0  # an earlier copy-bandwidth measurement on B200
 
 
 def hbm_peak() -> tuple[float, str]:
@@ -259,7 +276,7 @@ def hbm_peak() -> tuple[float, str]:
                 return float(v), "measured (MEASURED_PEAKS.json hbm_gbs)"
         except ValueError:
             pass
-    return HBM_FALLBACK_GBS, "fallback (6.65 TB/s, an earlier copy measurement on this pool)"
+    return HBM_FALLBACK_GBS, "fallback (6.65 TB/s, an earlier copy measurement)"
 
 
 def rank_window(rank: int, world: int, m_inc: int = WORKLOAD["m_inc"]) -> tuple[int, int]:
@@ -463,22 +480,20 @@ def run_ours(args, rank: int, world: int, local_rank: int, dist) -> dict | None:
     bits = (job.K * (m_start + m_inc // 2)).bit_length()
     limbs = job.info["limbs"]
     ppt_formula = products_per_test(bits)
-    one_thread = job.info["tpi"] == 1                  # persistent searches of one thread per number: k_search_tc
     ppt_mont = kernel_products_per_test(bits, limbs)
-    ppt = tc_products_per_test(bits, limbs) if one_thread else ppt_mont
+    kernel, ppt, ppt_what = search_work(job.info, bits, all(s["tc_blocks"] for s in stats))
     kern_s = kern_ms / 1e3
     peak = imad_peak / 2                               # a 32x32->64 product needs a lo and a hi multiply-add
     tr = traffic_per_launch()
-    work = (f"{ppt} limb products on the integer pipe per {bits}-bit test ({bits - 1} steps of {limbs} words: "
-            + ("L(L+1)/2 + 2L each; the reduction is two u8 matrix products on the tensor cores"
-               if one_thread else "L(L+1)/2 + L^2 + L each") + f"), {tests // args.steps} tests per launch; ")
+    work = (f"{ppt} limb products on the integer pipe per {bits}-bit test ({ppt_what}), "
+            f"{tests // args.steps} tests per launch; ")
     roof = {"bound": "imad", "achieved": tests * ppt / kern_s / 1e9, "peak": peak / 1e9,
             "unit": "G limb-products/s", "frac": tests * ppt / kern_s / peak,
             "frac_montgomery": tests * ppt_mont / kern_s / peak,
             "frac_formula": tests * ppt_formula / kern_s / peak,
             "traffic": tr.get("bytes_per_launch") if tr else None,
             "imad_pipe_busy_ncu": tr.get("imad_pipe_busy") if tr else None,
-            "kernel": f"k_search_{'tc' if one_thread else 'persistent_g'}<{limbs}>",
+            "kernel": kernel,
             "work": work + f"frac_montgomery counts the {ppt_mont} products of Montgomery squarings instead, "
                     f"frac_formula the fixed 2*L^2*(B+ceil(B/5)) = {ppt_formula}",
             "peak_source": "in-run microbenchmark (pg_measure_imad_peak: 32-bit IMAD/s / 2); "

@@ -7,6 +7,7 @@
 #include "pg_search_group.cuh"
 #include "pg_tc_search.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 namespace pg {
@@ -61,7 +62,10 @@ uint32_t pick_limbs(uint32_t words) { return pick_layout(32 * words, 0); }
 // Bases run side by side while 16 lanes (or groups) per number still finish in
 // the time of one test: up to 16 384 tests of one thread each (22 words:
 // 2.05 ms for 16 and for 16 384 tests), or 18 944 lanes in groups (one warp per
-// SM quarter).  Few tests of more than 20 words take a group of lanes per
+// SM quarter).  They also do for as many numbers of more than 20 words as base 2
+// alone tests in groups, for those take the other bases in turn slower than one
+// thread does (1 025 primes of 25 words, 16 bases: 63.5 ms in turn in groups, 52 on
+// one thread each, 7.2 with base 2 in groups and the others side by side).  Few tests of more than 20 words take a group of lanes per
 // number; the layouts were timed against one thread per number:
 //   21 words 8 x 3: 1.58, 1.60, 1.79 ms at 64, 2 048, 4 096 tests (1.85 to 1.95)
 //   22 words 8 x 3: 1.66, 1.87, 2.53 ms at 2 048, 4 096, 8 192 tests (2.05 at each)
@@ -94,13 +98,15 @@ uint32_t pick_batch(uint32_t words, uint32_t n, uint32_t rounds, bool *side_by_s
         if (L == PG_LAYOUT_GROUP(8, 136) && tests <= 2368) return PG_LAYOUT_GROUP(16, 144);
         return L;
     }
-    *side_by_side = rounds > 1 && n <= 1024;
+    // numbers that base 2 alone tests in groups
+    const uint32_t few = words > 23 ? (words == 48 ? 4096 : words > 24 ? 64 * words : 0) : words > 20 ? 4096 : 0;
+    *side_by_side = rounds > 1 && n <= std::max(1024u, few);
     const uint32_t tests = *side_by_side ? 16 * n : n;
     // lanes of base 2 at a warp per number, the other bases in groups of T lanes
     const auto apart = [&](uint32_t T) { return *side_by_side && n * (32 + (rounds - 1) * T) <= 18944; };
-    if (words > 16 && words <= 23 && (words > 20 ? tests <= 4096 : apart(8))) return PG_LAYOUT_GROUP(8, 24);
-    if (words > 23 && words <= 47 && (words > 24 ? tests <= 64 * words : apart(16))) return PG_LAYOUT_GROUP(16, 48);
-    if (words == 48 && tests <= 4096) return PG_LAYOUT_GROUP(8, 64);
+    if (words > 16 && words <= 23 && (few ? tests <= few : apart(8))) return PG_LAYOUT_GROUP(8, 24);
+    if (words > 23 && words <= 47 && (few ? tests <= few : apart(16))) return PG_LAYOUT_GROUP(16, 48);
+    if (words == 48 && tests <= few) return PG_LAYOUT_GROUP(8, 64);
     return L;
 }
 
@@ -115,9 +121,10 @@ cudaError_t launch_prp_batch(uint32_t L, const uint32_t *cand, uint32_t words, u
     // thread per number from 25 words on: from a warp an SM (1 024 composites, 16
     // bases: 32 words 5.7 ms in turn, 6.6 side by side, 40 words 10.9 and 14.8; at 48
     // words the two spill); the widest groups: from two (74 composites of 144 words
-    // 101.8 and 109.9 ms).  The others run beside it as fast as after it.
+    // 101.8 and 109.9 ms).  The others run beside it as fast as after it.  More than
+    // 1 024 numbers on one thread are those whose base 2 runs in groups.
     const uint32_t lanes = L >> 16 ? L >> 16 : 1, warps = n * ((rounds - 1) * lanes + (lanes > 1 ? 32 : 1)) / 32;
-    const bool tested = side_by_side && (L == 48 || (L >= 28 && lanes == 1 && warps > 148) ||
+    const bool tested = side_by_side && (L == 48 || (L >= 28 && lanes == 1 && warps > 148) || (lanes == 1 && n > 1024) ||
                                          (L == PG_LAYOUT_GROUP(8, 160) && warps > 2 * 148));
     if (tested) {
         bool one = false;

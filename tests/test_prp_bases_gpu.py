@@ -74,6 +74,17 @@ def test_composites_cost_no_more_than_in_turn(pg, ctx, words, n):
     assert side <= 1.1 * in_turn + 0.02
 
 
+@pytest.mark.parametrize("words,n", [(20, 1025), (21, 1025), (23, 4096), (24, 1025), (25, 1025), (28, 1792), (32, 2048),
+                                     (47, 3008), (48, 4096)])
+def test_primes_cost_no_more_than_in_turn(pg, ctx, words, n):
+    """More numbers than groups take side by side, all prime, 16 bases, against 4 097, which take the bases in turn on
+    one thread each and no longer than fewer would: a tenth for the clocks."""
+    values = [2 ** max(x for x in MERSENNE if x < 32 * words - 1) - 1] * 4_097
+    side, out = _ms(pg, ctx, words, values[:n], 16)
+    assert (out == 16).all()
+    assert side <= 1.1 * _ms(pg, ctx, words, values, 16)[0]
+
+
 @pytest.mark.parametrize("words,n", SHAPES)
 def test_first_failing_base(pg, ctx, oracle, words, n):
     """Primes, composites, pseudoprimes of the first bases, tiny, even and zero numbers in one batch."""

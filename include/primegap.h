@@ -99,7 +99,10 @@ typedef struct {
     uint32_t sl;           /* search radius: candidates X in [-sl, sl] are sieved */
     uint64_t max_prime;    /* sieve limit: every prime <= max_prime (--max-prime * 1e6) */
     uint64_t max_m_inc;    /* largest window later passed to pg_search / pg_sieve_interval */
-    uint64_t max_m;        /* largest m that will be searched (sizes the limbs) */
+    uint64_t max_m;        /* largest m that will be searched (sizes the limbs).  Below 2^30 the
+                              faster paths apply: searches on the tensor cores (pg_job_info.tc_words)
+                              and lattices in the sieve, which work with 32-bit m; a search that
+                              crosses 2^30 is best split into two jobs there */
     uint32_t rounds;       /* strong-PRP bases per accepted prime: 1 = base 2 only
                               (the reference's ROUNDS, gpu_testing.cu:62); r > 1 confirms
                               every base-2 probable prime with bases 3, 5, ... */

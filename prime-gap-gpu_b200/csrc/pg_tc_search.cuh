@@ -42,12 +42,13 @@ __device__ __forceinline__ int tc_pick_window(const SearchArgs &a, uint32_t kspa
 }
 
 // What bounds it: the integer multiply pipe (L(L+1)/2 + 2L word products a
-// step, 65 % busy with four CTAs of L = 23 on an SM, 57 % with two of L = 22)
-// together with the register ports that the carry chains and column sums load
-// beside it; the tensor pipe is 9 % busy and DRAM idle.  At L = 23 a step takes
-// 2 228 SM-quarter cycles per warp with four CTAs on an SM (1 877 with the
-// matrix round trips left out), at L = 40 5 513 with two; a Montgomery squaring
-// with the reduction on the multiply pipe takes 3 600 and 12 400.  A step alone
+// step, over whole searches 53 % busy with two CTAs of L = 22 on an SM, 68 % with
+// three of L = 23 and 70 % with two of L = 40) together with the register ports
+// that the carry chains and column sums load beside it; the tensor pipe is 7 to
+// 10 % busy and DRAM idle.  In a loop of steps alone one takes 2 228 SM-quarter
+// cycles per warp at L = 23 with four CTAs on an SM (1 877 with the matrix round
+// trips left out), at L = 40 5 513 with two; a Montgomery squaring with the
+// reduction on the multiply pipe takes 3 600 and 12 400.  A step alone
 // takes 3 800 cycles (two matrix round trips, the carry chains), so as many
 // CTAs as TMEM and registers hold share an SM.  Searches of P = 257 .. 947
 // (12 .. 44 words) run 1.2 .. 2.2 times as fast as on the one-warp kernel,

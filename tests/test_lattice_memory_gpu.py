@@ -67,3 +67,42 @@ def test_server_lattices_give_way_to_tables(pg):
                 assert srv.stats()["resident_bytes"] - slots > 28 * primes
         st = srv.stats()
     assert st["tables_built"] == len(keys) and st["tables_evicted"] == 0
+
+
+def test_lattices_give_way_beside_searches_in_flight(pg):
+    """Another thread's windows keep their results while the lattices they read are freed between launches."""
+    import threading
+    a_args = dict(p=503, d=2190, sl=10_000, max_prime=1_000_000_000, max_m_inc=1_500, max_m=2_000_000)
+    b_args = dict(p=337, d=2310, sl=7_500, max_prime=1_000_000_000, max_m_inc=1_500, max_m=11_000_000,
+                  flags=pg.PG_JOB_COMPACT_WALK)
+    results, stop, errors = [], threading.Event(), []
+
+    def search(job):
+        try:
+            while not stop.is_set():
+                tickets = [job.submit(1_000_000, 1_500) for _ in range(2)]
+                results.extend(job.wait(t) for t in tickets)
+        except Exception as e:  # noqa: BLE001 -- reported by the main thread
+            errors.append(e)
+
+    torch.cuda.empty_cache()
+    fill = None
+    with pg.Job(**a_args) as a:
+        first = a.search(1_000_000, 1_500)
+        worker = threading.Thread(target=search, args=(a,))
+        worker.start()
+        try:
+            need = 12 * a.info["num_primes"] + 300_000_000
+            fill = torch.empty(_free() - need + 400_000_000, dtype=torch.uint8, device="cuda")
+            with pg.Job(**b_args) as b:
+                assert (b.search(10_000_000, 1_500).next_gap > 0).all()
+                while len(results) < 12 and not errors:
+                    stop.wait(0.05)
+        finally:
+            stop.set()
+            worker.join()
+            del fill
+            torch.cuda.empty_cache()
+    assert not errors and len(results) >= 12
+    for r in results:
+        assert np.array_equal(r.prev_gap, first.prev_gap) and np.array_equal(r.next_gap, first.next_gap)

@@ -1,8 +1,6 @@
 """Lane-group searches of few sides: the blocks that the rounds rule launches against every block that fits."""
 from __future__ import annotations
 
-import time
-
 import numpy as np
 import pytest
 
@@ -10,12 +8,9 @@ pytestmark = pytest.mark.gpu
 
 
 def _ms(pg, job, m_inc, flags):
-    runs = []
-    for _ in range(5):
-        t = time.perf_counter()
-        res = job.wait(job.submit(1_000_001, m_inc, flags=flags))
-        runs.append((time.perf_counter() - t) * 1e3)
-    return sorted(runs)[1], res
+    """Device time of the window's kernels, best of five."""
+    runs = [job.wait(job.submit(1_000_001, m_inc, flags=flags)) for _ in range(5)]
+    return min(r.stats["total_ms"] for r in runs), runs[0]
 
 
 @pytest.mark.parametrize("P,d,tpi,m_inc", [(337, 2310, 16, 1_000), (337, 2310, 8, 1_400), (503, 2190, 8, 1_000),
